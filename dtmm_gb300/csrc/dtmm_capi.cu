@@ -26,6 +26,7 @@
 #include "../../include/dtmm_gb300.h"
 #include "dtmm_effmed.h"
 #include "dtmm_kernels.cuh"
+#include "dtmm_linekern.cuh"
 #include "dtmm_regkern.cuh"
 
 using namespace dtmm;
@@ -409,6 +410,33 @@ struct Prof {
 };
 enum { PROF_ROW = 0, PROF_COL = 1, PROF_OP = 2 };
 
+// launch shape of a line pass (dtmm_linekern.cuh) of `lines` n-point lines a block
+LineLaunch line_launch_of(const LineShape& ls, int lines, cudaStream_t st) {
+  LineLaunch L;
+  L.geom = LineGeom{ls.n1, ls.n2, ls.n2 | 1};
+  L.maxl = ls.maxl;
+  L.threads = std::max(64, (lines * std::max(ls.n1, ls.n2) + 31) / 32 * 32);
+  L.smem = 0;
+  L.st = st;
+  L.lim = 1 << 14;
+  return L;
+}
+
+// shared bytes of the scale words of `lines` fixed-point lines
+size_t part_bytes(int lines) {
+  return (size_t)lines * kPartPitch * sizeof(unsigned);
+}
+
+// plain complex128 row transforms through the line kernels
+cudaError_t launch_rows_line(const LineShape& ls, const void* src, void* dst, int nlines, int W, bool inv,
+                             const void* tw, double scale, cudaStream_t st) {
+  const int lpb = std::min((ls.maxl <= 16 ? 128 : 256) / std::max(ls.n1, ls.n2), 16);
+  LineLaunch L = line_launch_of(ls, lpb, st);
+  L.grid = dim3((unsigned)((nlines + lpb - 1) / lpb));
+  L.smem = ((size_t)lpb * ls.n1 * L.geom.pitch + W) * sizeof(cpx<double>) + part_bytes(lpb);
+  return rows_line(L, src, dst, nlines, W, inv, tw, scale, lpb);
+}
+
 template <typename R>
 struct Engine {
   Prof* prof = nullptr;
@@ -505,6 +533,10 @@ struct Engine {
   // the block whose effective medium the k-space tables fetched now use
   int cur_blk = 0;
 
+  // the line kernels take this side (fft_schedule 2 and 3 ask for the shared-memory passes)
+  bool line_on(int n) const { return sizeof(R) == 8 && d.fft_schedule <= 1 && line_shape(n).maxl > 0; }
+  bool row_line_on() const { return !row_reg() && line_on(d.width); }
+
   int launch_rows(cpx<R>* data, int C, bool inv, double scale) {
     const int nlines = NI * C * d.height;
     if constexpr (sizeof(R) == 4) {
@@ -520,6 +552,12 @@ struct Engine {
         if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_fft_rows_reg: %s", cudaGetErrorString(e));
         return DTMM_OK;
       }
+    }
+    if (line_on(d.width)) {
+      const cudaError_t e = launch_rows_line(line_shape(d.width), data, data, nlines, d.width, inv, P(L.twW), scale, st);
+      ++launches;
+      if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_rows_line: %s", cudaGetErrorString(e));
+      return DTMM_OK;
     }
     int lpb = 4096 / d.width;
     if (lpb < 1) lpb = 1;
@@ -570,20 +608,7 @@ struct Engine {
       RegLaunch rl;
       rl.smem = tiles * d.height * (C * tx + 1) * sizeof(cpx<R>) + d.height * sizeof(cpx<R>);
       rl.threads = std::max(32, ((C * tx * n1 + 31) / 32) * 32);
-      const int ntile = (d.width + tx - 1) / tx;
-      p.tile_lo = 0;
-      p.tile_hi0 = 0;
-      int nlaunch = ntile;
-      if (p.band_skip == 2 && p.kop == KOP_DIAG && blim_max >= 0) {
-        // tiles holding a column with |frequency index| <= the largest band limit
-        const int lo = (blim_max + 1 + tx - 1) / tx;        // columns 0 .. lim
-        const int hi0 = std::max(lo, (d.width - blim_max) / tx);  // columns W - lim .. W - 1
-        if (lo + (ntile - hi0) < ntile) {
-          p.tile_lo = lo;
-          p.tile_hi0 = hi0;
-          nlaunch = lo + (ntile - hi0);
-        }
-      }
+      const int nlaunch = band_tiles(p, tx);
       rl.grid = dim3(nlaunch, NI);
       rl.st = st;
       mark(PROF_COL);
@@ -597,14 +622,60 @@ struct Engine {
     }
   }
 
+  // column pass through the line kernels
+  int launch_col_line(ColParams& p, const cpx<R>* in, cpx<R>* out) {
+    const LineShape ls = line_shape(d.height);
+    const int cm = std::max(p.cin, p.cout), nmax = std::max(ls.n1, ls.n2);
+    const size_t per = (size_t)cm * d.height * sizeof(cpx<R>) * (p.ny > 1 ? 2 : 1);
+    const int most = ls.maxl <= 16 ? 128 : 256;  // the kernel's launch bounds
+    int tx = std::max(1, most / (cm * nmax));
+    while (tx > 1 && per * tx > 72 * 1024) tx /= 2;
+    // enough blocks for every SM
+    while (tx > 1 && (size_t)((d.width + tx - 1) / tx) * NI < 304) tx /= 2;
+    if (d.col_tile > 0 && d.col_tile * cm * nmax <= most && per * d.col_tile <= 180 * 1024) tx = d.col_tile;
+    tx = std::min(std::min(tx, d.width), kLineMax / cm);
+    if (per * tx + d.height * sizeof(cpx<R>) > 220 * 1024)
+      return fail(DTMM_ENOTSUP, "column of %d pixels too large for one block", d.height);
+    p.tc = tx;
+    LineLaunch rl = line_launch_of(ls, cm * tx, st);
+    rl.smem = per * tx + d.height * sizeof(cpx<R>) + part_bytes(cm * tx);
+    rl.lim = std::max(0, std::min(blimH_max, d.height));
+    const int nlaunch = band_tiles(p, tx);
+    rl.grid = dim3(nlaunch, NI);
+    mark(PROF_COL);
+    const cudaError_t e = col_line(rl, p, g, in, out);
+    mark(PROF_COL);
+    ++launches;
+    if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_col_line: %s", cudaGetErrorString(e));
+    return DTMM_OK;
+  }
+
+  // tiles of tx columns to launch: with band_skip 2 those holding a column
+  // with |frequency index| <= the largest band limit (p.tile_lo / tile_hi0)
+  int band_tiles(ColParams& p, int tx) const {
+    const int ntile = (d.width + tx - 1) / tx;
+    p.tile_lo = 0;
+    p.tile_hi0 = 0;
+    if (p.band_skip == 2 && p.kop == KOP_DIAG && blim_max >= 0) {
+      const int lo = (blim_max + 1 + tx - 1) / tx;              // columns 0 .. lim
+      const int hi0 = std::max(lo, (d.width - blim_max) / tx);  // columns W - lim .. W - 1
+      if (lo + (ntile - hi0) < ntile) {
+        p.tile_lo = lo;
+        p.tile_hi0 = hi0;
+        return lo + (ntile - hi0);
+      }
+    }
+    return ntile;
+  }
+
   int launch_col(const cpx<R>* in, cpx<R>* out, int cin, int cout, int kop, const void* ktab, int ny,
                  const R* cy, bool do_fwd, bool inverse_out, double scale, size_t ktab_ray_stride = 0,
                  int j_only = -1) {
     ColParams p;
     p.ktab_ray_stride = ktab_ray_stride;
-    // the engine's diagonal tables are cut at d.betamax; the register row
-    // pass reads out-of-band columns as zero, so skipped tiles need no writes
-    p.band_skip = row_reg() ? 2 : 1;
+    // the engine's diagonal tables are cut at d.betamax; the register and line
+    // row passes read out-of-band columns as zero, so skipped tiles need no writes
+    p.band_skip = row_reg() || row_line_on() ? 2 : 1;
     p.blim = blim();
     p.j_only = j_only;
     p.cy_rows = L.ny;
@@ -622,6 +693,8 @@ struct Engine {
     p.perm = A<int>(L.permH);
     const int cm = cin > cout ? cin : cout;
     if (col_reg() && cin == cout) return launch_col_reg(p, in, out, cin);
+    // (after shared-memory row passes the out-of-band columns have to be written)
+    if (line_on(d.height) && p.band_skip == 2) return launch_col_line(p, in, out);
     p.tc = tile_cols(cm, true);
     const size_t smem = 2 * (size_t)cm * d.height * p.tc * sizeof(cpx<R>) + d.height * (sizeof(cpx<R>) + sizeof(int));
     CK(cudaFuncSetAttribute(k_layer_col<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -723,6 +796,37 @@ struct Engine {
     }
   }
 
+  // row pass through the line kernels: about 8 lines a block
+  int launch_row_line(RowParams& p, const cpx<R>* Ub, cpx<R>* Xb, int C, bool re) {
+    const LineShape ls = line_shape(d.width);
+    const int nmax = std::max(ls.n1, ls.n2), most = ls.maxl <= 16 ? 128 : 256;
+    const size_t line_bytes = 2 * (size_t)ls.n1 * line_row_pitch(ls, re) * sizeof(cpx<R>);
+    p.PB = d.npol;
+    if (p.PB * C * nmax > most || p.PB * C * line_bytes > 200 * 1024 || p.PB * C > kLineMax) p.PB = 1;
+    const int perG = p.PB * C;
+    int G = std::max(1, std::min(8 / perG, most / (perG * nmax)));
+    if (d.row_group > 0) G = d.row_group;
+    while (G > 1 && ((size_t)G * perG * line_bytes > 100 * 1024 || G * perG * nmax > most || G * perG > kLineMax)) --G;
+    p.G = std::min(G, d.nlam);
+    const int nl = p.G * perG;
+    LineLaunch rl = line_launch_of(ls, nl, st);
+    rl.smem = nl * line_bytes + d.width * sizeof(cpx<R>) + part_bytes(nl);
+    if (rl.smem > 220 * 1024) return fail(DTMM_ENOTSUP, "row of %d pixels too large for one block", d.width);
+    const int ngrp = (d.nlam + p.G - 1) / p.G, npg = (d.npol + p.PB - 1) / p.PB;
+    // one layer's operator records beyond half of L2: the groups of a row next to each other
+    const size_t rec_bytes = (re ? sizeof(R) : sizeof(cpx<R>)) * (size_t)d.nray * L.nwin * p.rec_stride * L.HW;
+    p.groups_inner = rec_bytes > ((size_t)64 << 20) ? 1 : 0;
+    p.xr = 0;
+    rl.lim = std::max(0, std::min(blim_max, d.width));
+    rl.grid = p.groups_inner ? dim3(d.nray * ngrp * npg, d.height) : dim3(d.height, d.nray * ngrp * npg);
+    mark(PROF_ROW);
+    const cudaError_t e = row_line(C, re, rl, p, g, Ub, Xb);
+    mark(PROF_ROW);
+    ++launches;
+    if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_row_line: %s", cudaGetErrorString(e));
+    return DTMM_OK;
+  }
+
   int launch_row(const cpx<R>* Ub, cpx<R>* Xb, const void* op, double dir, int win_only = -1, bool use_cx = true,
                  bool accumulate = false) {
     RowParams p;
@@ -754,6 +858,7 @@ struct Engine {
         p.PB = 1;
       return launch_row_reg(p, Ub, Xb, L.C, re);
     }
+    if (row_line_on()) return launch_row_line(p, Ub, Xb, L.C, re);
     p.G = row_group();
     if (2 * (size_t)d.npol * L.C * (d.width | 1) * sizeof(cpx<R>) > 200 * 1024) p.PB = 1;
     if (L.C == 4) return re ? launch_row_t<4, true>(p, Ub, Xb) : launch_row_t<4, false>(p, Ub, Xb);
@@ -891,7 +996,7 @@ struct Engine {
     OpParams p;
     memset(&p, 0, sizeof(p));
     p.eps_dev = effb(blk_of(layer));
-    p.permW = row_reg() ? nullptr : A<int>(L.permW);
+    p.permW = row_reg() || row_line_on() ? nullptr : A<int>(L.permW);
     p.epsv = d.epsv;
     p.epsa = d.epsa;
     for (int i = 0; i < 3; ++i) {

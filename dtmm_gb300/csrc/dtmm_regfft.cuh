@@ -71,6 +71,22 @@ __host__ __device__ constexpr double sin2pi(long long n, long long d) { return c
 
 }  // namespace ct
 
+// cos / sin(2 pi n / d) as constants of the number type R
+template <typename R>
+struct CtConst {
+  static __host__ __device__ constexpr R cos2pi(long long n, long long d) { return (R)ct::cos2pi(n, d); }
+  static __host__ __device__ constexpr R sin2pi(long long n, long long d) { return (R)ct::sin2pi(n, d); }
+};
+
+// v (c + i s), a constant turn that is no quarter (eighth: by an odd number of eighths)
+template <typename R>
+struct RotGeneral {
+  template <bool EIGHTH>
+  static __host__ __device__ __forceinline__ cpx<R> run(cpx<R> v, R c, R s) {
+    return mk<R>(v.re * c - v.im * s, v.re * s + v.im * c);
+  }
+};
+
 // v * exp(s 2 pi i E / N), s = -1 forward, +1 inverse
 template <typename R, long long E, long long N, bool INV>
 __host__ __device__ __forceinline__ cpx<R> rotc(cpx<R> v) {
@@ -84,9 +100,9 @@ __host__ __device__ __forceinline__ cpx<R> rotc(cpx<R> v) {
   } else if constexpr (4 * e == 3 * N) {
     return INV ? mk<R>(v.im, -v.re) : mk<R>(-v.im, v.re);
   } else {
-    constexpr R c = (R)ct::cos2pi(e, N);
-    constexpr R s = INV ? (R)ct::sin2pi(e, N) : (R)-ct::sin2pi(e, N);
-    return mk<R>(v.re * c - v.im * s, v.re * s + v.im * c);
+    constexpr R c = CtConst<R>::cos2pi(e, N);
+    constexpr R s = INV ? CtConst<R>::sin2pi(e, N) : -CtConst<R>::sin2pi(e, N);
+    return RotGeneral<R>::template run<(8 * e) % N == 0>(v, c, s);
   }
 }
 
@@ -96,8 +112,8 @@ __host__ __device__ __forceinline__ cpx<R> rotc(cpx<R> v) {
 template <typename R, int P, bool INV, int S, int J>
 __host__ __device__ __forceinline__ void prime_acc(const cpx<R>* x, cpx<R>& a, cpx<R>& b) {
   if constexpr (J <= (P - 1) / 2) {
-    constexpr R c = (R)ct::cos2pi((long long)J * S, P);
-    constexpr R s = (R)ct::sin2pi((long long)J * S, P);
+    constexpr R c = CtConst<R>::cos2pi((long long)J * S, P);
+    constexpr R s = CtConst<R>::sin2pi((long long)J * S, P);
     const cpx<R> sp = x[J] + x[P - J], dm = x[J] - x[P - J];
     a = mk<R>(a.re + c * sp.re, a.im + c * sp.im);
     b = mk<R>(b.re + s * dm.re, b.im + s * dm.im);

@@ -1,0 +1,60 @@
+"""Fixed-point line passes (complex128 bulk) against the FP64 shared-memory
+passes of the same library (``fft_schedule`` 2): every side with kernels of its
+own, run-time sides of both length classes, the smallest and the largest, the
+4x4 method with windows and the 2x2 one.
+
+Tolerance: two layers are about 20 transforms and products of relative error
+below 5e-16, and phases of at most 10 rad rounded at 2^-53: 2e-14 together.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(64, 64), (80, 96), (100, 120), (128, 150), (160, 144), (180, 192), (225, 240), (256, 256), (7, 2), (5, 16),
+          (45, 50), (200, 330), (250, 125), (512, 300), (24, 1024)]
+
+
+def _run(shape, method, diffraction, schedule, spoil=None, scale=1.0):
+    import torch
+
+    from dtmm_gb300 import samples
+    from dtmm_gb300.illumination import illumination_device
+    from dtmm_gb300.transfer import plan_transfer
+
+    wl = [450.0, 620.0]
+    mat = samples.twisted_nematic_device(shape, 2, no=1.52, ne=1.71, amplitude=0.3, seed=5)
+    fin = illumination_device(shape, wl, 100.0, beta=0.1, phi=0.4, precision="double") * scale
+    if spoil is not None:
+        fin[0, 1, 0, shape[0] // 2, shape[1] // 2] = spoil
+    plan = plan_transfer(tuple(fin.shape), wl, 100.0, mat, beta=0.1, phi=0.4, method=method, diffraction=diffraction,
+                         npass=1, precision="double", tuning=dict(fft_schedule=schedule))
+    out = torch.empty_like(fin)
+    plan.run(fin, out)
+    return out.cpu().numpy()
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("method,diffraction", [("4x4", 3), ("2x2", 1)])
+def test_line_passes_match_fp64_passes(shape, method, diffraction):
+    a = _run(shape, method, diffraction, 0)
+    b = _run(shape, method, diffraction, 2)
+    assert np.linalg.norm(a - b) <= 2e-14 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("scale", [1e-120, 1e120])
+def test_line_passes_scale(scale):
+    # the line's own power of two: the result is the scaled result to rounding
+    a = _run((64, 50), "4x4", 3, 0)
+    b = _run((64, 50), "4x4", 3, 0, scale=scale) / scale
+    assert np.linalg.norm(a - b) <= 2e-14 * np.linalg.norm(a)
+
+
+@pytest.mark.parametrize("spoil", [np.nan, np.inf])
+def test_line_passes_not_finite(spoil):
+    # one bad value: its image is lost, as in FP64 arithmetic, and no other one is touched
+    a = _run((64, 50), "4x4", 3, 0, spoil=spoil)
+    b = _run((64, 50), "4x4", 3, 2, spoil=spoil)
+    assert not np.isfinite(a[0, 1]).any() and not np.isfinite(b[0, 1]).any()
+    for i in ((0, 0), (1, 0), (1, 1)):
+        assert np.linalg.norm(a[i] - b[i]) <= 2e-14 * np.linalg.norm(b[i])
