@@ -94,78 +94,88 @@ __host__ __device__ __forceinline__ float to_r<float>(double d) {
   return f32_rn(d);
 }
 
-#ifdef __CUDACC__
 // An FP32 value widened to FP64 exactly, in integer arithmetic (normal
 // floats; others take the hardware conversion, which issues at the FP64 rate)
-__device__ __forceinline__ double f64_of(float f) {
+__host__ __device__ __forceinline__ double f64_of(float f) {
+#ifdef __CUDA_ARCH__
   const unsigned b = __float_as_uint(f);
   const unsigned e = (b >> 23) & 0xffu;
   if (e == 0u || e == 0xffu) return (double)f;
   const unsigned long long u = ((unsigned long long)(b & 0x80000000u) << 32) |
                                ((unsigned long long)(e + 896u) << 52) | ((unsigned long long)(b & 0x7fffffu) << 29);
   return __longlong_as_double((long long)u);
+#else
+  return (double)f;
+#endif
 }
 
-// Square root of x > 0 for results stored in FP32: the FP32 reciprocal square
-// root of x (its input truncated to FP32 in integer arithmetic) refined by
-// one Newton-Raphson step for 1/sqrt(x), y <- y (3 - x y^2) / 2, whose error
-// is about 1.5 e^2 for a seed error e (<= 1e-6 here, so <= 2e-12), then
-// sqrt(x) = x y: five FP64 operations.  Arguments outside the float range
-// (and non-positive ones) take the library square root.
-__device__ __forceinline__ double sqrt_pos_fast(double x) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-  const unsigned hi = (unsigned)(u >> 32);
-  const int e = (int)((hi >> 20) & 0x7ffu) - 896;  // FP32 biased exponent
-  if ((hi & 0x80000000u) || e < 2 || e > 252) return sqrt(x);
-  const float xf = __uint_as_float(((unsigned)e << 23) | ((hi & 0xfffffu) << 3) | ((unsigned)u >> 29));
-  const double y0 = f64_of(rsqrtf(xf));
-  const double hy = (0.5 * x) * y0;
-  const double y = y0 * fma(-hy, y0, 1.5);
-  return x * y;
+// ---------------------------------------------------------------------------
+// Pairs of FP32 numbers, h + l with |l| a few last places of h at most: about
+// 46 bits at FP32 rates (Dekker, "A floating-point technique for extending the
+// available precision", 1971; products by FMA).  Every sum and product is
+// rounded on its own (no contraction).
+// ---------------------------------------------------------------------------
+struct ff {
+  float h, l;
+};
+__host__ __device__ __forceinline__ ff ff_mk(float h, float l) {
+  ff r;
+  r.h = h;
+  r.l = l;
+  return r;
+}
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ float f_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float f_mul(float a, float b) { return __fmul_rn(a, b); }
+#else
+inline float f_add(float a, float b) { return a + b; }
+inline float f_mul(float a, float b) { return a * b; }
+#endif
+__host__ __device__ __forceinline__ float ff_f(ff a) { return f_add(a.h, a.l); }
+__host__ __device__ __forceinline__ ff ff_of(double x) {
+  const float h = f32_rn(x);
+  return ff_mk(h, f32_rn(x - f64_of(h)));
+}
+__host__ __device__ __forceinline__ ff ff_add(ff a, ff b) {
+  const float s = f_add(a.h, b.h), t = f_add(s, -a.h);
+  const float e = f_add(f_add(a.h, -f_add(s, -t)), f_add(b.h, -t));
+  return ff_mk(s, f_add(e, f_add(a.l, b.l)));
+}
+__host__ __device__ __forceinline__ ff ff_sub(ff a, ff b) { return ff_add(a, ff_mk(-b.h, -b.l)); }
+__host__ __device__ __forceinline__ ff ff_mul(ff a, ff b) {
+  const float p = f_mul(a.h, b.h);
+  return ff_mk(p, fmaf(a.h, b.l, fmaf(a.l, b.h, fmaf(a.h, b.h, -p))));
+}
+// sqrt(a), a > 0 (an FP32 root for a <= 0): one Newton step on the remainder
+__host__ __device__ __forceinline__ ff ff_sqrt(ff a) {
+  if (!(a.h > 0.0f)) return ff_mk(sqrtf(ff_f(a)), 0.0f);
+#ifdef __CUDA_ARCH__
+  const float y = rsqrtf(a.h);
+#else
+  const float y = 1.0f / sqrtf(a.h);
+#endif
+  const float r = f_mul(a.h, y);
+  return ff_mk(r, f_mul(f_add(fmaf(-r, r, a.h), a.l), f_mul(0.5f, y)));
+}
+// a / b: the quotient of the high parts and its remainder's
+__host__ __device__ __forceinline__ ff ff_div(ff a, ff b) {
+#ifdef __CUDA_ARCH__
+  const float y = __frcp_rn(b.h);
+#else
+  const float y = 1.0f / b.h;
+#endif
+  const float q = f_mul(a.h, y);
+  const float r = fmaf(-q, b.l, f_add(fmaf(-q, b.h, a.h), a.l));
+  return ff_mk(q, f_mul(r, y));
+}
+// v / 2^62, |v| <= 2^62
+__host__ __device__ __forceinline__ ff ff_q62(long long v) {
+  const int hi = (int)(v >> 38);
+  const int lo = (int)((v - ((long long)hi << 38)) >> 7);
+  return ff_mk((float)hi * 5.9604644775390625e-8f, (float)lo * 2.7755575615628914e-17f);  // 2^-24, 2^-55
 }
 
-// Square root of x > 0 in three FP64 operations from an FP32 seed: with y0
-// the FP32 reciprocal square root of x (input truncated to FP32 in integer
-// arithmetic), r0 = x y0, hy0 = y0 / 2 and e = x - r0^2, sqrt(x) is
-// fma(hy0, e, r0): one Newton-Raphson step for the square root, relative
-// error about 1.5 s^2 for a seed error s (<= 3e-7 here, so <= 2e-13).  The
-// parts are returned so that a caller can fold a term into the last fma.
-// Arguments outside the float range, and non-positive ones, take the library
-// square root (r0 = sqrt(x), hy0 = e = 0).
-__device__ __forceinline__ void sqrt_newton(double x, double& r0, double& hy0, double& e) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-  const unsigned hi = (unsigned)(u >> 32);
-  const int ex = (int)((hi >> 20) & 0x7ffu) - 896;  // FP32 biased exponent
-  if ((hi & 0x80000000u) || ex < 2 || ex > 252) {
-    r0 = sqrt(x);
-    hy0 = 0.0;
-    e = 0.0;
-    return;
-  }
-  const float xf = __uint_as_float(((unsigned)ex << 23) | ((hi & 0xfffffu) << 3) | ((unsigned)u >> 29));
-  const float yf = rsqrtf(xf);
-  r0 = x * f64_of(yf);
-  hy0 = f64_of(0.5f * yf);
-  e = fma(-r0, r0, x);
-}
-
-// 1 / x for a normal x from the FP32 reciprocal of x (input truncated to FP32
-// in integer arithmetic) and two Newton-Raphson steps y <- y + y (1 - x y):
-// four FP64 operations; the seed error (<= 2e-7) squares twice, so the result
-// is within a few FP64 roundings of 1 / x.
-// Arguments outside the float range take the FP64 division.
-__device__ __forceinline__ double rcp_newton(double x) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-  const unsigned hi = (unsigned)(u >> 32);
-  const int ex = (int)((hi >> 20) & 0x7ffu) - 896;
-  if (ex < 2 || ex > 252) return 1.0 / x;
-  const float xf = __uint_as_float((hi & 0x80000000u) | ((unsigned)ex << 23) | ((hi & 0xfffffu) << 3) |
-                                   ((unsigned)u >> 29));
-  double y = f64_of(__frcp_rn(xf));
-  y = fma(y, fma(-x, y, 1.0), y);
-  return fma(y, fma(-x, y, 1.0), y);
-}
-
+#ifdef __CUDACC__
 // d == 0 (either sign), in integer arithmetic
 __device__ __forceinline__ bool is_zero_d(double d) { return (__double_as_longlong(d) << 1) == 0; }
 #endif

@@ -11,7 +11,9 @@
 
 #include "dtmm_common.cuh"
 #include "dtmm_eig4.cuh"
+#include "dtmm_fx.cuh"
 #include "dtmm_layer.cuh"
+#include "dtmm_lean.cuh"
 
 namespace dtmm {
 
@@ -238,30 +240,35 @@ __device__ __forceinline__ bool voxel_E_real(double beta, const VoxelInv& vi, do
 }
 
 // Lean solve for complex64 records (real eps above beta^2, uniaxial or
-// isotropic voxels): the per-(ray, window) constants of the launch sit in
-// shared memory (beam terms beta cos phi, beta sin phi; with one eps for
-// every voxel eps11 - beta^2, its square root, eps11 (eps11 - beta^2 +
-// delta) and the ordinary mode's phase record), and per voxel and window the
-// eigenvalues of dtmm/tmm.py:157-278 take about 12 FP64 operations (16 with
-// the backward modes):
-//   gamma = beta cos(az - phi) = cos(az) beta cos(phi) + sin(az) beta sin(phi)
-//   q = u c2 - eps11 kw gamma^2   (a quarter of the discriminant v^2 - 4 u w,
-//                                  whose delta^2 terms cancel)
-//   alpha+- = (-kvh gamma +- sqrt(q)) / u   (kvh = delta sin(t) cos(t); sqrt
-//                                  from an FP32 seed and one Newton step)
-// FP64 because the phase records (alpha - a_w) d cancel.  The E entries,
-// which the records keep in FP32, are formed in FP32 from the FP32-rounded
-// eigenvalue and voxel / beam terms (sin(t) folded into the cos / sin of
-// (az - phi)), rotated back by phi, and their determinants formed and
-// inverted in FP32: each entry within a few FP32 roundings of its FP64 value.
+// isotropic voxels) in pairs of FP32 numbers (48 bits, dtmm_common.cuh).  FP64
+// issues at 1/64 of the FP32 rate here: the same eigenvalues at 12 FP64
+// operations a voxel and window kept that pipe 87 % busy and took 0.86 ms for
+// 1024 x 1024 voxels and 25 windows; a pair operation costs 4 to 8 FP32 ones.
+//
+// The records hold (alpha - a_w) d, formed without cancellation (dtmm_lean.cuh).
+//
+// The E entries, which the records keep in FP32, are formed in FP32 from the
+// rounded eigenvalue and voxel / beam terms (sin(t) folded into the cos / sin
+// of (az - phi)), rotated back by phi, and their determinants formed and
+// inverted in FP32.  The launch's per-(ray, window) constants sit in shared
+// memory; the angles' sines and cosines come from the integer turns of
+// dtmm_fx.cuh (the library's FP64 sincos of two angles would cost as much as
+// six windows).
 struct LeanWin {
-  double beta, cp, sp, bcp, bsp;  // beam: beta, cos / sin phi, beta cos / sin phi
-  double ev02, evs, c2;           // one eps for every voxel: eps11 - beta^2, its root, eps11 (ev02 + delta)
-  double awd;                     // a_w d
-  float cpf, spf, r6;             // cos / sin phi in FP32; (evs - a_w) d (one eps for every voxel)
-  float betaf, ev02f, evsf;       // beta, and with one eps for every voxel ev02, evs, in FP32
+  ff a, bcp, bsp, c2, b2;           // a_w, beta cos / sin phi, with one eps c2, beta^2
+  float betaf, cpf, spf;            // beta, cos / sin phi
+  float r6, ev02f, evsf;            // with one eps: (evs - a_w) d, eps11 - beta^2, its root
 };
 constexpr int kLeanChunk = 32;  // windows per shared-memory chunk (<= the block size)
+
+// cos and sin of an angle as pairs
+__device__ __forceinline__ void ff_sincos(double ang, ff& s, ff& c) {
+  const double u = ang * 0.15915494309189533577;
+  const cpx<fx> t = fx_turn(u);
+  s = ff_q62(t.im.v);
+  c = ff_q62(t.re.v);
+  if ((fx_hiword(u) & 0x7ff00000) == 0x7ff00000) s.h = c.h = __int_as_float(0x7fc00000);
+}
 
 template <bool FOUR>
 __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, float* __restrict__ opv, int pix,
@@ -273,35 +280,32 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
   const bool active = pix < HW;
   const bool uni = p.wev02 != nullptr;
   // the voxel's invariants, shared by every ray and window
-  double e0 = 0.0, delta = 0.0, ie = 0.0, iu = 0.0, ct = 0.0, ca = 0.0, sa = 0.0, sca = 0.0, ssa = 0.0;
-  double kvh = 0.0, qb = 0.0, u = 0.0;
-  float caf = 0.0f, saf = 0.0f, scaf = 0.0f, ssaf = 0.0f, ctf = 0.0f, ief = 0.0f;  // FP32 copies for E
+  const ff z = ff_mk(0.0f, 0.0f);
+  LeanVoxel vx = {};
+  ff e0 = z, e2 = z, n0 = z;
+  float caf = 0.0f, saf = 0.0f, ctf = 0.0f, scaf = 0.0f, ssaf = 0.0f, ief = 0.0f;  // FP32 copies for E
   bool iso = false;
   size_t slot = 0;
+  const ff dd = ff_of(p.d);
   if (active) {
     const int y = pix / g.W, x = pix - y * g.W;
     const long long eo = p.layer * p.ev_s[0] + y * p.ev_s[1] + x * p.ev_s[2];
     const long long ao = p.layer * p.ea_s[0] + y * p.ea_s[1] + x * p.ea_s[2];
     const double* e = (const double*)p.epsv + eo;
-    e0 = e[0];
-    iso = e[0] == e[1] && e[1] == e[2];
-    delta = e[2] - e[0];
-    double st;
-    sincos(p.epsa[ao + 1], &st, &ct);
-    sincos(p.epsa[ao + 2], &sa, &ca);
-    ie = rcp_newton(e0);
-    u = fma(delta, ct * ct, e0);
-    iu = rcp_newton(u);
-    kvh = delta * (st * ct);
-    qb = e0 * (delta * (st * st));
-    sca = st * ca;
-    ssa = st * sa;
-    caf = f32_rn(ca);
-    saf = f32_rn(sa);
-    scaf = f32_rn(sca);
-    ssaf = f32_rn(ssa);
-    ctf = f32_rn(ct);
-    ief = f32_rn(ie);
+    const double eo0 = e[0], ee = e[2], eps = p.uncorrected ? 0.0 : p.eps_dev[0];
+    iso = eo0 == e[1] && e[1] == ee;
+    ff_sincos(p.epsa[ao + 1], vx.st, vx.ct);
+    ff_sincos(p.epsa[ao + 2], vx.sa, vx.ca);
+    e0 = ff_of(eo0);
+    e2 = ff_of(ee);
+    n0 = ff_of(eo0 - eps);
+    lean_voxel(vx, e0, ff_of(ee - eo0), ff_of(eo0 * (ee - eps)));
+    caf = ff_f(vx.ca);
+    saf = ff_f(vx.sa);
+    ctf = ff_f(vx.ct);
+    scaf = ff_f(ff_mul(vx.st, vx.ca));
+    ssaf = ff_f(ff_mul(vx.st, vx.sa));
+    ief = ff_f(ff_div(ff_mk(1.0f, 0.0f), e0));
     slot = (size_t)y * g.W + (p.permW ? p.permW[x] : x);
   }
   const int rw0 = ray0 * p.nwin, rw1 = ray1 * p.nwin;
@@ -311,26 +315,22 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
     if ((int)threadIdx.x < n) {
       const int rw = c0 + threadIdx.x;
       LeanWin w;
-      w.beta = p.wbeta[rw];
-      w.cp = p.wcos[rw];
-      w.sp = p.wsin[rw];
-      w.bcp = w.beta * w.cp;
-      w.bsp = w.beta * w.sp;
+      const double beta = p.wbeta[rw], cp = p.wcos[rw], sp = p.wsin[rw];
       const double aw = p.uncorrected ? 0.0 : p.waw[rw];
-      w.awd = aw * p.d;
-      w.cpf = f32_rn(w.cp);
-      w.spf = f32_rn(w.sp);
-      w.betaf = f32_rn(w.beta);
+      w.a = ff_of(aw);
+      w.bcp = ff_of(beta * cp);
+      w.bsp = ff_of(beta * sp);
+      w.b2 = ff_of(beta * beta);
+      w.betaf = f32_rn(beta);
+      w.cpf = f32_rn(cp);
+      w.spf = f32_rn(sp);
+      w.c2 = z;
+      w.r6 = w.ev02f = w.evsf = 0.0f;
       if (uni) {
-        w.ev02 = p.wev02[rw];
-        w.evs = p.wevs[rw];
-        w.c2 = p.wc2[rw];
-        w.r6 = f32_rn((w.evs - aw) * p.d);
-        w.ev02f = f32_rn(w.ev02);
-        w.evsf = f32_rn(w.evs);
-      } else {
-        w.ev02 = w.evs = w.c2 = 0.0;
-        w.r6 = w.ev02f = w.evsf = 0.0f;
+        w.c2 = ff_of(p.wc2[rw]);
+        w.r6 = f32_rn((p.wevs[rw] - aw) * p.d);
+        w.ev02f = f32_rn(p.wev02[rw]);
+        w.evsf = f32_rn(p.wevs[rw]);
       }
       wc[threadIdx.x] = w;
     }
@@ -338,59 +338,48 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
     if (!active) continue;
     for (int k = 0; k < n; ++k) {
       const LeanWin& w = wc[k];
-      double ev02, evs, c2;
-      float r6, ev02f, evsf;
-      if (uni) {
-        ev02 = w.ev02;
-        evs = w.evs;
-        c2 = w.c2;
-        r6 = w.r6;
-        ev02f = w.ev02f;
-        evsf = w.evsf;
-      } else {
-        ev02 = e0 - w.beta * w.beta;
-        evs = sqrt_pos_fast(ev02);
-        c2 = e0 * (ev02 + delta);
-        r6 = f32_rn(fma(evs, p.d, -w.awd));
-        ev02f = f32_rn(ev02);
-        evsf = f32_rn(evs);
+      float r6 = w.r6, ev02f = w.ev02f, evsf = w.evsf;
+      ff c2 = w.c2;
+      if (!uni) {
+        const ff x = ff_sub(e0, w.b2), ev = ff_sqrt(x);
+        c2 = ff_mul(e0, ff_sub(e2, w.b2));
+        r6 = ff_f(ff_mul(ff_div(p.uncorrected ? x : n0, ff_add(ev, w.a)), dd));
+        ev02f = ff_f(x);
+        evsf = ff_f(ev);
       }
       // E rows (Ex, Ey) of the forward modes 0, 2 (backward 1, 3), in the beam
-      // frame, in FP32; the eigenvalues in FP64
+      // frame, and their phase records
       float E00, E10, E02, E12, E01 = 0.0f, E11 = 0.0f, E03 = 0.0f, E13 = 0.0f;
-      double al0, al1 = 0.0;
+      float r4 = r6, r10 = -r6;
       bool zero = false;
       if (iso) {
-        al0 = evs;
-        al1 = -evs;
         E00 = 0.5f; E10 = 0.0f; E02 = 0.0f; E12 = 0.5f;
         if (FOUR) { E01 = 0.5f; E11 = 0.0f; E03 = 0.0f; E13 = 0.5f; }
-        zero = evs == 0.0;
-      } else if (w.beta == 0.0) {
-        const float cf = fmaf(caf, w.cpf, saf * w.spf), sf = fmaf(saf, w.cpf, -caf * w.spf);
-        const double sq = sqrt(u * c2) * iu;
-        al0 = sq;
-        al1 = -sq;
-        E00 = cf; E10 = sf; E02 = -evsf * sf; E12 = evsf * cf;
-        if (FOUR) { E01 = cf; E11 = sf; E03 = E02; E13 = E12; }
+        zero = evsf == 0.0f;
       } else {
-        const double gama = fma(ca, w.bcp, sa * w.bsp);
-        const double q = fma(-qb, gama * gama, u * c2);
-        double r0, hy0, eq;
-        sqrt_newton(q, r0, hy0, eq);
-        const double kvg = kvh * gama;
-        al0 = fma(hy0, eq, r0 - kvg) * iu;
-        const float a0f = f32_rn(al0);
-        const float cfst = fmaf(scaf, w.cpf, ssaf * w.spf), sfst = fmaf(ssaf, w.cpf, -scaf * w.spf);
-        const float ctbeta = ctf * w.betaf;
-        const float ev02cf = ev02f * cfst;
-        E00 = fmaf(a0f, ctbeta, -ev02cf) * ief;  E10 = -sfst;
-        E02 = evsf * sfst;                       E12 = fmaf(-evsf, cfst, ctbeta);
+        ff dp, dm;
+        lean_roots<FOUR>(vx, w.a, w.bcp, w.bsp, c2, p.uncorrected ? c2 : vx.cv, dp, dm);
+        r4 = ff_f(ff_mul(dp, dd));
+        const float a0f = w.a.h + (w.a.l + (dp.h + dp.l));
+        float a1f = 0.0f;
         if (FOUR) {
-          al1 = -fma(hy0, eq, r0 + kvg) * iu;
-          const float a1f = f32_rn(al1);
-          E01 = fmaf(-a1f, ctbeta, ev02cf) * ief;  E11 = sfst;
-          E03 = -E02;                              E13 = fmaf(evsf, cfst, ctbeta);
+          r10 = ff_f(ff_mul(dm, dd));
+          a1f = -w.a.h + ((dm.h + dm.l) - w.a.l);
+        }
+        if (w.betaf == 0.0f) {
+          const float cf = fmaf(caf, w.cpf, saf * w.spf), sf = fmaf(saf, w.cpf, -caf * w.spf);
+          E00 = cf; E10 = sf; E02 = -evsf * sf; E12 = evsf * cf;
+          if (FOUR) { E01 = cf; E11 = sf; E03 = E02; E13 = E12; }
+        } else {
+          const float cfst = fmaf(scaf, w.cpf, ssaf * w.spf), sfst = fmaf(ssaf, w.cpf, -scaf * w.spf);
+          const float ctbeta = ctf * w.betaf;
+          const float ev02cf = ev02f * cfst;
+          E00 = fmaf(a0f, ctbeta, -ev02cf) * ief;  E10 = -sfst;
+          E02 = evsf * sfst;                       E12 = fmaf(-evsf, cfst, ctbeta);
+          if (FOUR) {
+            E01 = fmaf(-a1f, ctbeta, ev02cf) * ief;  E11 = sfst;
+            E03 = -E02;                              E13 = fmaf(evsf, cfst, ctbeta);
+          }
         }
       }
       const float df = fmaf(E00, E12, -(E02 * E10));
@@ -409,7 +398,7 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
         rec[1] = ex2 * w.cpf - ey2 * w.spf;
         rec[2] = (ex0 * w.spf + ey0 * w.cpf) * sf;
         rec[3] = ex2 * w.spf + ey2 * w.cpf;
-        rec[4] = iso ? r6 : f32_rn(fma(al0, p.d, -w.awd));
+        rec[4] = r4;
         rec[5] = r6;
         if (FOUR) {
           const float ex1 = E01, ey1 = E11, ex3 = E03, ey3 = E13;
@@ -418,7 +407,7 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
           rec[7] = ex3 * w.cpf - ey3 * w.spf;
           rec[8] = (ex1 * w.spf + ey1 * w.cpf) * sb;
           rec[9] = ex3 * w.spf + ey3 * w.cpf;
-          rec[10] = iso ? -r6 : f32_rn(fma(al1, p.d, w.awd));
+          rec[10] = r10;
           rec[11] = -r6;
         }
       }
