@@ -410,6 +410,15 @@ struct Prof {
 };
 enum { PROF_ROW = 0, PROF_COL = 1, PROF_OP = 2 };
 
+// launch shape of the register column pass of `lines` n-point lines a block
+RegLaunch col_reg_shape(int n, int lines, cudaStream_t st) {
+  RegLaunch rl;
+  rl.threads = std::max(32, (lines * col_threads_per_line(n) + 31) / 32 * 32);
+  rl.smem = col_smem(n, lines);
+  rl.st = st;
+  return rl;
+}
+
 // launch shape of a line pass (dtmm_linekern.cuh) of `lines` n-point lines a block
 LineLaunch line_launch_of(const LineShape& ls, int lines, cudaStream_t st) {
   LineLaunch L;
@@ -537,7 +546,11 @@ struct Engine {
   bool line_on(int n) const { return sizeof(R) == 8 && d.fft_schedule <= 1 && line_shape(n).maxl > 0; }
   bool row_line_on() const { return !row_reg() && line_on(d.width); }
 
+  // the buffer that holds a row pass's band-limited output, if any
+  const cpx<R>* row_out = nullptr;
+
   int launch_rows(cpx<R>* data, int C, bool inv, double scale) {
+    if (data == row_out) row_out = nullptr;
     const int nlines = NI * C * d.height;
     if constexpr (sizeof(R) == 4) {
       if (d.fft_schedule <= 1 && reg_lanes(d.width) > 0) {
@@ -589,31 +602,19 @@ struct Engine {
   // register-transform column pass: complex64 bulk, sides listed by reg_lanes
   bool col_reg() const { return sizeof(R) == 4 && d.fft_schedule <= 1 && reg_lanes(d.height) > 0; }
 
-  int launch_col_reg(ColParams& p, const cpx<R>* in, cpx<R>* out, int C) {
+  int launch_col_reg(ColParams& p, const cpx<R>* in, cpx<R>* out) {
     if constexpr (sizeof(R) != 4) {
       return fail(DTMM_ENOTSUP, "register column transform is complex64 only");
     } else {
-      const int n1 = reg_lanes(d.height);
-      const size_t tiles = reg_col_tiles(d.height, p.ny);
-      int tx = std::max(1, 256 / (C * n1));
-      // tiles of H x (C tx + 1) complex: about 3 blocks per SM by default
-      size_t cap = tiles == 2 ? 72 * 1024 : 100 * 1024;
-      if (d.col_tile > 0 && d.col_tile * C * n1 <= 256) {  // the kernel's launch bound
-        tx = d.col_tile;
-        cap = 160 * 1024;
-      }
-      if (tx > d.width) tx = d.width;
-      while (tx > 1 && tiles * d.height * (C * tx + 1) * sizeof(cpx<R>) > cap) tx /= 2;
-      p.tc = tx;
-      RegLaunch rl;
-      rl.smem = tiles * d.height * (C * tx + 1) * sizeof(cpx<R>) + d.height * sizeof(cpx<R>);
-      rl.threads = std::max(32, ((C * tx * n1 + 31) / 32) * 32);
-      const int nlaunch = band_tiles(p, tx);
-      rl.grid = dim3(nlaunch, NI);
-      rl.st = st;
+      const int cm = std::max(p.cin, p.cout);
+      int tx = kColLines / cm;
+      if (d.col_tile > 0) tx = std::min(tx, d.col_tile);
+      p.tc = tx = std::min(tx, d.width);
+      RegLaunch rl = col_reg_shape(d.height, cm * tx, st);
+      rl.grid = dim3(band_tiles(p, tx), NI);
       mark(PROF_COL);
-      // the diagonal table is cut at betamax: band variants of the inverse transforms
-      const int band = p.kop == KOP_DIAG ? row_band_pick(d.height, blimH_max) : 0;
+      // the diagonal table is cut at betamax: band variants of the transforms
+      const int band = p.kop == KOP_DIAG && p.do_fwd && p.inverse_out ? col_band_pick(d.height, blimH_max) : 0;
       const cudaError_t e = col_reg_dispatch(d.height, band, rl, p, g, in, out);
       mark(PROF_COL);
       ++launches;
@@ -677,6 +678,8 @@ struct Engine {
     // row passes read out-of-band columns as zero, so skipped tiles need no writes
     p.band_skip = row_reg() || row_line_on() ? 2 : 1;
     p.blim = blim();
+    p.xband = in == row_out ? 1 : 0;
+    if (out == row_out) row_out = nullptr;
     p.j_only = j_only;
     p.cy_rows = L.ny;
     p.cin = cin;
@@ -692,7 +695,7 @@ struct Engine {
     p.tw = P(L.twH);
     p.perm = A<int>(L.permH);
     const int cm = cin > cout ? cin : cout;
-    if (col_reg() && cin == cout) return launch_col_reg(p, in, out, cin);
+    if (col_reg()) return launch_col_reg(p, in, out);
     // (after shared-memory row passes the out-of-band columns have to be written)
     if (line_on(d.height) && p.band_skip == 2) return launch_col_line(p, in, out);
     p.tc = tile_cols(cm, true);
@@ -834,6 +837,10 @@ struct Engine {
     p.win_only = win_only;
     p.use_cx = use_cx ? 1 : 0;
     p.accumulate = accumulate ? 1 : 0;
+    // a k-space operator that is zero beyond betamax follows every row pass
+    // with diffraction (chains copy their results, ret_bulk transforms them)
+    p.band_out = d.diffraction >= 1 && !L.chains && io.bulk == nullptr && (row_reg() || row_line_on()) ? 1 : 0;
+    row_out = p.band_out ? Xb : nullptr;
     p.PB = d.npol;
     p.C = L.C;
     p.nx = L.nx;
@@ -1601,6 +1608,7 @@ struct Engine {
     const cpx<R>* t2;
     if ((rc = table(KT_D2, dir * dprev / 2, t2))) return rc;
     if ((rc = launch_col(cur, U, 4, 4, KOP_MAT, t2, 1, nullptr, true, true, 1.0 / d.height))) return rc;
+    row_out = nullptr;
     if ((rc = launch_rows(U, 4, true, 1.0 / d.width))) return rc;
     CK(cudaMemcpyAsync(F, U, sizeof(cpx<R>) * (size_t)NI * 4 * L.HW, cudaMemcpyDeviceToDevice, st));
     return DTMM_OK;
@@ -2071,6 +2079,7 @@ struct Engine {
         if ((rc = launch_rows(U, 4, true, iw))) return rc;
         if ((rc = axpby(fin, fin, nullptr, 1.0, U, nullptr, 1.0))) return rc;
       }
+      row_out = nullptr;
     }
     return DTMM_OK;
   }
@@ -2487,17 +2496,9 @@ int diffract_impl(int H, int W, int nimg, int nlam, const void* dmat, const void
   p.perm = permH;
   if (sizeof(R) == 4 && reg_lanes(H) > 0) {
     // register column transforms with the matrix exchanged through the tile
-    const int n1 = reg_lanes(H);
-    const size_t tiles = reg_col_tiles(H, 1);
-    int tx = std::max(1, 256 / (4 * n1));
-    if (tx > W) tx = W;
-    while (tx > 1 && tiles * H * (4 * tx + 1) * sizeof(cpx<R>) > 100 * 1024) tx /= 2;
-    p.tc = tx;
-    RegLaunch cl;
-    cl.smem = tiles * H * (4 * tx + 1) * sizeof(cpx<R>) + H * sizeof(cpx<R>);
-    cl.threads = std::max(32, ((4 * tx * n1 + 31) / 32) * 32);
-    cl.grid = dim3((W + tx - 1) / tx, nimg);
-    cl.st = st;
+    p.tc = std::min(kColLines / 4, W);
+    RegLaunch cl = col_reg_shape(H, 4 * p.tc, st);
+    cl.grid = dim3((W + p.tc - 1) / p.tc, nimg);
     const cudaError_t e = col_reg_dispatch(H, 0, cl, p, g, X, out);
     ++launches;
     if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_layer_col_reg: %s", cudaGetErrorString(e));

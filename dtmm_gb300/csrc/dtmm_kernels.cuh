@@ -2284,7 +2284,8 @@ __global__ void __launch_bounds__(256) k_layer_col(ColParams p, Grid g, const cp
     const int c = t / (H * TC), r = t - c * H * TC;
     const int y = r / TC, xc = r - y * TC;
     const int x = x0 + xc;
-    cpx<R> v = (x < W) ? X[(((size_t)img * p.cin + c) * H + y) * W + x] : mk<R>(0, 0);
+    const bool live = x < W && (!p.xband || (x < (W + 1) / 2 ? x : W - x) <= (int)p.blim[lam]);
+    cpx<R> v = live ? X[(((size_t)img * p.cin + c) * H + y) * W + x] : mk<R>(0, 0);
     const int ys = p.do_fwd ? perm[y] : y;
     T[((size_t)ys * CM + c) * TC + xc] = v;
   }

@@ -75,6 +75,10 @@ struct ColParams {
   // 1: such tiles write zeros; 2: they write nothing (the register row pass
   // reads those columns as zero without loading them)
   int band_skip;
+  // 1: the input is a row pass's band-limited output (RowParams::band_out):
+  // columns beyond the band are unwritten and read as zeros, and the k-space
+  // operator is zero there; tiles of such columns become zeros at once
+  int xband;
   const double* blim;      // [lam] band limit: largest in-band |column frequency index| (-1: none)
   int tile_lo, tile_hi0;   // register column pass with band_skip 2: launched tiles [0, tile_lo) and
                            // tile_hi0 on (tile_lo 0: every tile)
@@ -116,6 +120,7 @@ struct RowParams {
   int win_only;          // >= 0: only this window (its own sub-step chain), -1: all
   int use_cx;            // apply the window's beta_x weight (first sub-step of a chain)
   int accumulate;        // add the result to X instead of overwriting it
+  int band_out;          // 1: columns beyond the band need not be written (ColParams::xband reads them as zeros)
   int groups_inner;      // register row pass: blockIdx.x the group, blockIdx.y the row (else the reverse)
   int xr;                // register row pass variant with accumulators in registers, pixels a thread (0: none)
 };

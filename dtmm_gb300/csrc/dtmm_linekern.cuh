@@ -249,6 +249,8 @@ __global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
 #pragma unroll
           for (int m = 0; m < MAXL; ++m) {
             if (m >= len) break;
+            // band_out: the next column pass reads the columns inside the band only
+            if (p.band_out && m > limW / n1 && m < (W - limW) / n1) continue;
             const cpx<double> r = line_out(v[m], emax, guard);
             dst[n1 * m] = p.accumulate ? dst[n1 * m] + r : r;
           }
@@ -395,14 +397,24 @@ __global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
   const int x0 = tile * TX;
   const int lam = img_lam(g, img), ray = img_ray(g, img);
   const bool diag = p.kop == KOP_DIAG;
-  if (p.band_skip == 2 && diag) {  // tiles beyond the band: nothing is read from them
+  bool band_x = true;  // the thread's column is read
+  if ((p.band_skip == 2 && diag) || p.xband) {  // tiles beyond the band: nothing is read from them, or zeros
     const int lim = (int)p.blim[lam];
     bool any = false;
     for (int xc = 0; xc < TX && x0 + xc < W; ++xc) {
       const int xk = x0 + xc;
       any = any || (xk < (W + 1) / 2 ? xk : W - xk) <= lim;
     }
-    if (!any) return;
+    const int line = threadIdx.x % NL, c = line / TX, kx = x0 + line - c * TX;
+    if (!any) {
+      if (!diag && c < p.cout && kx < W)
+        for (int jj = 0; jj < p.ny; ++jj) {
+          cpx<double>* udst = U + ((size_t)jj * g.NI * p.cout + (size_t)img * p.cout + c) * H * W + kx;
+          for (int y = threadIdx.x / NL; y < H; y += blockDim.x / NL) udst[(size_t)y * W] = mk<double>(0.0, 0.0);
+        }
+      return;
+    }
+    if (p.xband) band_x = (kx < (W + 1) / 2 ? kx : W - kx) <= lim;
   }
   cpx<fx>* tile_x = (cpx<fx>*)smem_raw;                                    // [H][NL] exchange
   cpx<double>* tile_s = (cpx<double>*)(p.ny > 1 ? tile_x + (size_t)H * NL : tile_x);  // [H][NL] spectra along y
@@ -439,7 +451,7 @@ __global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
 #pragma unroll
           for (int m = 0; m < MAXL; ++m) {
             if (m >= len) break;
-            d[m] = in_x ? src[(size_t)(t + n2 * m) * W] : mk<double>((double)0, (double)0);
+            d[m] = in_x && band_x ? src[(size_t)(t + n2 * m) * W] : mk<double>(0.0, 0.0);
           }
         } else {
           const double* cyj = p.cy ? (const double*)p.cy + (((size_t)ray * p.cy_rows + j) * g.nlam + lam) * H : nullptr;
@@ -511,7 +523,7 @@ __global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
           const int ak = k < (H + 1) / 2 ? k : H - k;
           cpx<double> a = mk<double>((double)0, (double)0);
           if (!diag || ak <= limH) {
-            a = skip_dft ? (in_x ? src[(size_t)k * W] : a) : line_out(v[m], emax, guard);
+            a = skip_dft ? (in_x && band_x ? src[(size_t)k * W] : a) : line_out(v[m], emax, guard);
             if (ek) a = a * ek[(size_t)k * 2];
             if (p.kop != KOP_MAT) a = a * sc;
           }

@@ -9,13 +9,9 @@
 //                the line's row buffer, the per-voxel operator accumulates into
 //                the line's accumulator, and the accumulator is transformed
 //                forward and stored (natural order throughout);
-//   column pass  TX columns x C components of one image: coalesced row loads
-//                into a tile, forward column transforms, the diagonal k-space
-//                operator, then per window row j: spectra * cy_j -> inverse
-//                transform -> coalesced row stores.  With N2 % N1 == 0 the
-//                spectra stay in registers and one tile serves as loads,
-//                exchange and stores; otherwise they stay in tile A and the
-//                exchange uses tile B (A itself for a single window row).
+//   column pass  TX columns x C components of one image: forward column
+//                transforms, the k-space operator, then per window row j:
+//                spectra * cy_j -> inverse transform (k_layer_col_reg).
 //
 // The kernels are instantiated per side in separate translation units
 // (dtmm_reg_*.cu) through DTMM_REG_DEFINE; the engine reaches them through the
@@ -281,16 +277,22 @@ __global__ void __launch_bounds__(XR > 0 ? (N1 * N2) / (XR > 0 ? XR : 1) : (N2 >
     cpx<R> u[TS::J][N1];
     TS::template step2<R, false>(u, xl, 1, t);
     cpx<R>* dst = X + (((size_t)img * C + c) * H + y) * W;
+    constexpr int KBO = row_band_slots(N2, BAND);
     if constexpr (TS::EVEN) {
       TS::template to_lane_order<R>(u, v);
 #pragma unroll
-      for (int m = 0; m < N2; ++m) dst[t + N1 * m] = p.accumulate ? dst[t + N1 * m] + v[m] : v[m];
+      for (int m = 0; m < N2; ++m) {
+        // band_out: the next column pass reads the columns inside the band only
+        if (BAND != 0 && m >= KBO && m < N2 - KBO && p.band_out) continue;
+        dst[t + N1 * m] = p.accumulate ? dst[t + N1 * m] + v[m] : v[m];
+      }
     } else {
       __syncwarp(gm);
       TS::template store<R>(u, xl, 1, t, (R)1);
       __syncwarp(gm);
 #pragma unroll
       for (int m = 0; m < N2; ++m) {
+        if (BAND != 0 && m >= KBO && m < N2 - KBO && p.band_out) continue;
         const cpx<R> r = xl[t + N1 * m];
         dst[t + N1 * m] = p.accumulate ? dst[t + N1 * m] + r : r;
       }
@@ -340,42 +342,75 @@ __global__ void __launch_bounds__(256) k_fft_rows_reg(const cpx<R>* src, cpx<R>*
   }
 }
 
-// tiles of the column pass: N2 % N1 == 0 keeps the spectra in registers (one
-// tile); otherwise the spectra stay in tile A and, with several window rows,
-// the exchange needs tile B
-__host__ __device__ constexpr bool reg_even(int n) { return reg_lanes(n) > 0 && (n / reg_lanes(n)) % reg_lanes(n) == 0; }
-__host__ __device__ constexpr int reg_col_tiles(int n, int ny) { return (!reg_even(n) && ny > 1) ? 2 : 1; }
+// Split of the column pass, n = n1 n2: the most even one (up to 32 each).
+__host__ __device__ constexpr int col_n1(int n) {
+  int best = 0;
+  for (int a = 1; a * a <= n; ++a)
+    if (n % a == 0 && n / a <= 32) best = a;
+  return best;
+}
+__host__ __device__ constexpr int col_pitch(int n) { return (n / col_n1(n)) | 1; }
+__host__ __device__ constexpr int col_threads_per_line(int n) { return n / col_n1(n); }
+// lines of a block at most: tiles of four columns of four components
+constexpr int kColLines = 16;
+__host__ __device__ constexpr size_t col_smem(int n, int lines) {
+  return ((size_t)lines * col_n1(n) * col_pitch(n) + n) * 2 * sizeof(float);
+}
+// threads of a block at most (whole warps), and blocks a SM: 24 warps while
+// that leaves 80 registers a thread
+__host__ __device__ constexpr int col_max_threads(int n) { return (kColLines * col_threads_per_line(n) + 31) / 32 * 32; }
+__host__ __device__ constexpr int col_min_blocks(int n) {
+  return 768 / col_max_threads(n) > 1 ? 768 / col_max_threads(n) : 1;
+}
+// band variant of an n-point column for the largest band limit (as row_band_pick)
+__host__ __device__ constexpr int col_band_pick(int n, int lim) {
+  const int n1 = col_n1(n), n2 = n / n1;
+  for (int b = 1; b <= 2; ++b)
+    if (row_band_ok(n2, b) && lim < row_band_slots(n2, b) * n1) return b;
+  return 0;
+}
 
-// Column pass, k-space operator KOP_NONE, KOP_DIAG or KOP_MAT (C x C per k,
-// exchanged through the tile; see the file comment).  BAND > 0 (KOP_DIAG
-// only, N2 % N1 == 0): the diagonal table is zero beyond betamax, so after it
-// a lane's spectrum entries outside m < KB, m >= N2 - KB are exact zeros
-// whenever the H axis's band limit is below KB N1; the window-row inverse
-// transforms then weight only those entries and run the sparse step 1.
-template <typename R, int N1, int N2, int BAND>
-__global__ void __launch_bounds__(256, 3) k_layer_col_reg(ColParams p, Grid g, const cpx<R>* __restrict__ X,
-                                                         cpx<R>* __restrict__ U) {
-  using TS = TwoStep<N1, N2>;
-  constexpr int H = N1 * N2;
+// Column pass, complex64 bulk, k-space operator KOP_NONE, KOP_DIAG or KOP_MAT
+// (cin x cout per k).  TX columns x max(cin, cout) components of one image;
+// consecutive threads on consecutive columns, n2 (the larger factor) threads a
+// line.  A thread loads its points of the forward transform's first step from
+// global memory straight into registers and stores the inverse transform's
+// results from registers, so a line passes through shared memory once per
+// transform (exchange slots (k, s) at k + P s, P = n2 | 1, lines innermost):
+//   forward  t < n2: y = t + n2 m, DFT n1, twiddle  -> slots t + P k
+//            t < n1: slots s + P t, DFT n2          -> ky = t + n1 m, in registers
+//   inverse  t < n1: x cy_j, DFT n2, twiddle        -> slots k + P t
+//            t < n2: slots t + P s, DFT n1          -> y = t + n2 m
+// BAND > 0 (KOP_DIAG): the table is zero beyond betamax and the axis' band
+// limit is below KB n1, so only the entries m < KB and m >= n2 - KB exist: the
+// forward transform forms no others and the inverse one runs the sparse DFT.
+// Latency-bound (a launch is one to four waves of blocks); staging the columns
+// through shared memory on the way in and out, as before, took 27 us for 256
+// points (three window rows, 18 images), 249 us for 1024 (five rows, 6 images,
+// two components) and 121 us for 320 (70 images), this takes 20, 120 and 83.
+template <typename R, int N, int BAND>
+__global__ void __launch_bounds__(col_max_threads(N), col_min_blocks(N))
+    k_layer_col_reg(ColParams p, Grid g, const cpx<R>* __restrict__ X, cpx<R>* __restrict__ U) {
+  constexpr int H = N, N1 = col_n1(N), N2 = N / N1, P = N2 | 1;
+  constexpr bool D = BAND != 0;  // KOP_DIAG between two transforms: nothing else is compiled in
+  constexpr int KB = row_band_slots(N2, BAND);
+  constexpr unsigned MASK = BAND == 0 ? full_mask(N2) : band_mask(N2, KB);
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int W = g.W, TX = p.tc, C = p.cin;
-  const int RS = C * TX + 1;                       // tile row stride (odd)
-  const int ntiles = reg_col_tiles(H, p.ny);
-  cpx<R>* tileA = (cpx<R>*)smem_raw;               // [H][RS] loaded rows, then spectra along y
-  cpx<R>* tileB = tileA + (size_t)(ntiles - 1) * H * RS;  // [H][RS] exchange and outgoing rows (= A with one tile)
-  cpx<R>* tw = tileA + (size_t)ntiles * H * RS;    // [H] twiddles, lane-major (TwoStep::twiddle_entry)
+  const int W = g.W, TX = p.tc, CM = max(p.cin, p.cout), NL = CM * TX;
+  cpx<R>* tile = (cpx<R>*)smem_raw;         // [N1 P][NL]
+  cpx<R>* tw = tile + (size_t)N1 * P * NL;  // [H] W^(t k) at k N1 + t, t < N1
   const int img = blockIdx.y;
   // tile_lo > 0: the launch covers the in-band tiles only, tiles [0, tile_lo)
   // and from tile_hi0 on (the others write nothing with band_skip 2)
-  const int tile = (p.tile_lo > 0 && (int)blockIdx.x >= p.tile_lo) ? p.tile_hi0 + ((int)blockIdx.x - p.tile_lo)
-                                                                    : (int)blockIdx.x;
-  const int x0 = tile * TX;
+  const int bx = (p.tile_lo > 0 && (int)blockIdx.x >= p.tile_lo) ? p.tile_hi0 + ((int)blockIdx.x - p.tile_lo)
+                                                                  : (int)blockIdx.x;
+  const int x0 = bx * TX;
   const int lam = img_lam(g, img), ray = img_ray(g, img);
-  const int CT = C * TX;
-  const int lc = threadIdx.x % CT, ystep = blockDim.x / CT;
-  const int lcc = lc / TX, lxc = lc - lcc * TX;
-  const bool lin = (int)threadIdx.x < ystep * CT && x0 + lxc < W;
-  if (p.band_skip && p.kop == KOP_DIAG) {
+  const int line = threadIdx.x % NL, t = threadIdx.x / NL;
+  const int c = line / TX, kx = x0 + (line - c * TX);
+  const bool in_x = kx < W;
+  bool live = in_x;  // the column is read
+  if ((p.band_skip && p.kop == KOP_DIAG) || p.xband) {
     const int lim = (int)p.blim[lam];
     bool any = false;
     for (int xc = 0; xc < TX && x0 + xc < W; ++xc) {
@@ -383,182 +418,151 @@ __global__ void __launch_bounds__(256, 3) k_layer_col_reg(ColParams p, Grid g, c
       any = any || (xk < (W + 1) / 2 ? xk : W - xk) <= lim;
     }
     if (!any) {  // the whole block leaves together
-      if (p.band_skip == 1) {
-        for (int jj = 0; jj < p.ny; ++jj) {
-          cpx<R>* udst = U + (size_t)jj * g.NI * C * H * W + ((size_t)img * C + lcc) * H * W + x0 + lxc;
-          if (lin)
-            for (int y = threadIdx.x / CT; y < H; y += ystep) udst[(size_t)y * W] = mk<R>((R)0, (R)0);
-        }
+      if (p.band_skip == 1 || p.kop != KOP_DIAG) {
+        if (c < p.cout && in_x)
+          for (int jj = 0; jj < p.ny; ++jj) {
+            cpx<R>* udst = U + ((size_t)jj * g.NI * p.cout + (size_t)img * p.cout + c) * H * W + kx;
+            for (int y = t; y < H; y += blockDim.x / NL) udst[(size_t)y * W] = mk<R>((R)0, (R)0);
+          }
       }
       return;
     }
+    if (p.xband) live = in_x && (kx < (W + 1) / 2 ? kx : W - kx) <= lim;
   }
-  for (int e = threadIdx.x; e < H; e += blockDim.x) tw[e] = TS::twiddle_entry((const cpx<R>*)p.tw, e);
-  const cpx<R>* xsrc = X + ((size_t)img * C + lcc) * H * W + x0 + lxc;
-  if (lin)
-    for (int y = threadIdx.x / CT; y < H; y += ystep) tileA[y * RS + lc] = xsrc[(size_t)y * W];
-  __syncthreads();
-  const int l = threadIdx.x / N1, t = threadIdx.x % N1;
-  const int nlines = C * TX;
-  const bool active = l < nlines;
-  const unsigned gm = group_mask<N1>();
-  const int c = l / TX, xc = l - c * TX;
-  const int kx = x0 + xc;
-  cpx<R>* colA = tileA + l;  // line element e at colA[e * RS]
-  cpx<R>* colB = tileB + l;
-  const bool diag = active && p.kop == KOP_DIAG && kx < W;
-  const cpx<R>* ek = diag ? (const cpx<R>*)p.ktab + (((size_t)lam * W + kx) * H) * 2 + ((((c & 1) == 0) || C == 2) ? 0 : 1)
-                          : nullptr;
+  cpx<R> v[N2];
+  if (D || p.do_fwd) {
+    // (loads first: the twiddle table fills while they are in flight)
+    cpx<R> u[N1];
+    const bool act = t < N2 && c < p.cin;
+    if (act) {
+      const cpx<R>* src = X + (((size_t)img * p.cin + c) * H + t) * W + kx;
+#pragma unroll
+      for (int m = 0; m < N1; ++m) {
+        u[m] = live ? *src : mk<R>((R)0, (R)0);
+        src += N2 * W;
+      }
+    }
+    for (int e = threadIdx.x; e < H; e += blockDim.x) tw[e] = ((const cpx<R>*)p.tw)[(e % N1) * (e / N1)];
+    __syncthreads();
+    if (act) {
+      RegDFTg<R, N1, false>::run(u);
+      tile[(size_t)t * NL + line] = u[0];
+#pragma unroll
+      for (int k = 1; k < N1; ++k) tile[(size_t)(t + P * k) * NL + line] = u[k] * tw[t * N1 + k];
+    }
+    __syncthreads();
+    if (t < N1 && c < p.cin) {
+#pragma unroll
+      for (int m = 0; m < N2; ++m) v[m] = tile[(size_t)(m + P * t) * NL + line];
+      RegDFTg<R, N2, false>::run(v);
+    }
+  } else {
+    for (int e = threadIdx.x; e < H; e += blockDim.x) tw[e] = ((const cpx<R>*)p.tw)[(e % N1) * (e / N1)];
+    if (t < N1 && c < p.cin) {
+      const cpx<R>* src = X + (((size_t)img * p.cin + c) * H + t) * W + kx;
+#pragma unroll
+      for (int m = 0; m < N2; ++m) {
+        v[m] = live ? *src : mk<R>((R)0, (R)0);
+        src += N1 * W;
+      }
+    }
+    __syncthreads();
+  }
   const R sc = (R)p.out_scale;
-  if constexpr (TS::EVEN) {
-    // spectra in registers, lane order v[m] = X[t + N1 m]
-    cpx<R> v[N2];
-    if (active) {
+  if (!D && p.kop == KOP_MAT) {
+    // the matrix per k across a column's components, one point a turn, through the thread's own slots
+    if (t < N1 && c < p.cin) {
 #pragma unroll
-      for (int m = 0; m < N2; ++m) v[m] = colA[(t + N1 * m) * RS];
-      __syncwarp(gm);
-      if (p.do_fwd) {
-        TS::template step1<R, false>(v, colA, RS, nullptr, tw, t);
-        __syncwarp(gm);
-        cpx<R> u[TS::J][N1];
-        TS::template step2<R, false>(u, colA, RS, t);
-        TS::template to_lane_order<R>(u, v);
-      }
-      if (diag) {
+      for (int m = 0; m < N2; ++m) tile[(size_t)(m + P * t) * NL + line] = v[m];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < H * TX; e += blockDim.x) {
+      const int k = e / TX, xe = e - k * TX, kt = k % N1, km = k / N1;
+      if (x0 + xe >= W) continue;
+      cpx<R>* z = tile + (size_t)(km + P * kt) * NL + xe;
+      const cpx<R>* mt = (const cpx<R>*)p.ktab + ray * p.ktab_ray_stride +
+                         (((size_t)lam * H + k) * W + x0 + xe) * p.cout * p.cin;
+      cpx<R> in[4];
 #pragma unroll
-        for (int m = 0; m < N2; ++m) v[m] = v[m] * ek[(t + N1 * m) * 2];
+      for (int i = 0; i < 4; ++i)
+        if (i < p.cin) in[i] = z[i * TX];
+#pragma unroll
+      for (int o = 0; o < 4; ++o) {
+        if (o >= p.cout) break;
+        cpx<R> a = mk<R>((R)0, (R)0);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (i < p.cin) a = cfma(mt[o * p.cin + i], in[i], a);
+        z[o * TX] = a * sc;
       }
-      // the output scale once on the spectrum, not on every window row's result
+    }
+    __syncthreads();
+    if (t < N1 && c < p.cout) {
+#pragma unroll
+      for (int m = 0; m < N2; ++m) v[m] = tile[(size_t)(m + P * t) * NL + line];
+    }
+  } else if (t < N1 && c < p.cin) {
+    if (D || p.kop == KOP_DIAG) {
+      if (in_x) {
+        const cpx<R>* ek = (const cpx<R>*)p.ktab + (((size_t)lam * W + kx) * H + t) * 2 +
+                           ((((c & 1) == 0) || p.cin == 2) ? 0 : 1);
+#pragma unroll
+        for (int m = 0; m < N2; ++m)
+          if (BAND == 0 || m < KB || m >= N2 - KB) v[m] = v[m] * (ek[(size_t)m * N1 * 2] * sc);
+      }
+    } else {
 #pragma unroll
       for (int m = 0; m < N2; ++m) v[m] = v[m] * sc;
     }
-    if (p.kop == KOP_MAT) {
-      // C x C matrix per k across the components of a column: through tile A
-      __syncthreads();  // every line's forward exchange is done with the tile
-      if (active) {
-#pragma unroll
-        for (int m = 0; m < N2; ++m) colA[(t + N1 * m) * RS] = v[m];
-      }
-      __syncthreads();
-      if (active && kx < W) {
-        const cpx<R>* mt = (const cpx<R>*)p.ktab + ray * p.ktab_ray_stride + (((size_t)lam * H) * W + kx) * C * C + c * C;
-#pragma unroll
-        for (int m = 0; m < N2; ++m) {
-          const int k = t + N1 * m;
-          const cpx<R>* mrow = mt + (size_t)k * W * C * C;
-          const cpx<R>* in = tileA + (size_t)k * RS + xc;
-          cpx<R> acc = mk<R>((R)0, (R)0);
-          for (int j = 0; j < C; ++j) acc = cfma(mrow[j], in[j * TX], acc);
-          v[m] = acc;
-        }
-      }
-    }
-    for (int jj = 0; jj < p.ny; ++jj) {
-      const int j = p.j_only >= 0 ? p.j_only : jj;
-      __syncthreads();  // the previous window's stores (and the forward exchange) are done with the tile
-      if (active) {
-        const R* cyj = p.cy ? (const R*)p.cy + (((size_t)ray * p.cy_rows + j) * g.nlam + lam) * H : nullptr;
-        constexpr int KB = row_band_slots(N2, BAND);
-        cpx<R> w[N2];
-#pragma unroll
-        for (int m = 0; m < N2; ++m) {
-          if (BAND == 0 || m < KB || m >= N2 - KB)
-            w[m] = cyj ? v[m] * cyj[t + N1 * m] : v[m];
-          else
-            w[m] = mk<R>((R)0, (R)0);
-        }
-        if (p.inverse_out) {
-          TS::template step1<R, true, BAND == 0 ? full_mask(N2) : band_mask(N2, KB)>(w, colA, RS, nullptr, tw, t);
-          __syncwarp(gm);
-          cpx<R> u[TS::J][N1];
-          TS::template step2<R, true>(u, colA, RS, t);
-          __syncwarp(gm);
-          TS::template store<R>(u, colA, RS, t);
-        } else {
-#pragma unroll
-          for (int m = 0; m < N2; ++m) colA[(t + N1 * m) * RS] = w[m];
-        }
-      }
-      __syncthreads();
-      cpx<R>* udst = U + (size_t)jj * g.NI * C * H * W + ((size_t)img * C + lcc) * H * W + x0 + lxc;
-      if (lin)
-        for (int y = threadIdx.x / CT; y < H; y += ystep) udst[(size_t)y * W] = tileA[y * RS + lc];
-    }
-  } else {
-    // spectra in tile A (natural order); exchange in tile B (tile A itself
-    // with one window row: the line is in registers before the exchange)
-    if (active && p.do_fwd) {
-      cpx<R> v[N2];
-#pragma unroll
-      for (int m = 0; m < N2; ++m) v[m] = colA[(t + N1 * m) * RS];
-      __syncwarp(gm);
-      TS::template step1<R, false>(v, colB, RS, nullptr, tw, t);
-      __syncwarp(gm);
-      cpx<R> u[TS::J][N1];
-      TS::template step2<R, false>(u, colB, RS, t);
-      __syncwarp(gm);
-      TS::template store<R>(u, colA, RS, t, (R)1);
-    }
-    if (diag) {
-      __syncwarp(gm);
+  }
+  for (int jj = 0; jj < p.ny; ++jj) {
+    const int j = p.j_only >= 0 ? p.j_only : jj;
+    cpx<R>* udst = U + ((size_t)jj * g.NI * p.cout + (size_t)img * p.cout + c) * H * W + kx;
+    if (t < N1 && c < p.cout) {
+      const R* cyj = p.cy ? (const R*)p.cy + (((size_t)ray * p.cy_rows + j) * g.nlam + lam) * H + t : nullptr;
+      cpx<R> w[N2];
 #pragma unroll
       for (int m = 0; m < N2; ++m) {
-        const int k = t + N1 * m;
-        colA[k * RS] = colA[k * RS] * ek[k * 2];
+        if (BAND == 0 || m < KB || m >= N2 - KB)
+          w[m] = cyj ? v[m] * cyj[N1 * m] : v[m];
+        else
+          w[m] = mk<R>((R)0, (R)0);
       }
-    }
-    if (p.kop == KOP_MAT) {
-      // C x C matrix per k across the components of a column, in tile A:
-      // every thread reads its k's components, the block syncs, then writes
-      __syncthreads();
-      cpx<R> r[N2];
-      if (active && kx < W) {
-        const cpx<R>* mt = (const cpx<R>*)p.ktab + ray * p.ktab_ray_stride + (((size_t)lam * H) * W + kx) * C * C + c * C;
+      if (D || p.inverse_out) {
+        RegDFTs<R, N2, true, MASK>::run(w);
+        tile[(size_t)P * t * NL + line] = w[0];
+#pragma unroll
+        for (int k = 1; k < N2; ++k) {
+          cpx<R> f = tw[k * N1 + t];
+          f.im = -f.im;
+          tile[(size_t)(k + P * t) * NL + line] = w[k] * f;
+        }
+      } else if (in_x) {
+        cpx<R>* o = udst + (size_t)t * W;
 #pragma unroll
         for (int m = 0; m < N2; ++m) {
-          const int k = t + N1 * m;
-          const cpx<R>* mrow = mt + (size_t)k * W * C * C;
-          const cpx<R>* in = tileA + (size_t)k * RS + xc;
-          cpx<R> acc = mk<R>((R)0, (R)0);
-          for (int j = 0; j < C; ++j) acc = cfma(mrow[j], in[j * TX], acc);
-          r[m] = acc;
+          *o = w[m];
+          o += N1 * W;
         }
-      }
-      __syncthreads();
-      if (active && kx < W) {
-#pragma unroll
-        for (int m = 0; m < N2; ++m) colA[(t + N1 * m) * RS] = r[m];
       }
     }
-    for (int jj = 0; jj < p.ny; ++jj) {
-      const int j = p.j_only >= 0 ? p.j_only : jj;
-      __syncthreads();  // tile A complete; the previous window's stores have read tile B
-      if (active) {
-        cpx<R> v[N2];
-        const R* cyj = p.cy ? (const R*)p.cy + (((size_t)ray * p.cy_rows + j) * g.nlam + lam) * H : nullptr;
+    if (!D && !p.inverse_out) continue;
+    __syncthreads();
+    if (t < N2 && c < p.cout) {
+      cpx<R> u[N1];
 #pragma unroll
-        for (int m = 0; m < N2; ++m) {
-          const cpx<R> a = colA[(t + N1 * m) * RS];
-          v[m] = cyj ? a * cyj[t + N1 * m] : a;
-        }
-        __syncwarp(gm);
-        if (p.inverse_out) {
-          TS::template step1<R, true>(v, colB, RS, nullptr, tw, t);
-          __syncwarp(gm);
-          cpx<R> u[TS::J][N1];
-          TS::template step2<R, true>(u, colB, RS, t);
-          __syncwarp(gm);
-          TS::template store<R>(u, colB, RS, t, sc);
-        } else {
+      for (int m = 0; m < N1; ++m) u[m] = tile[(size_t)(t + P * m) * NL + line];
+      RegDFTg<R, N1, true>::run(u);
+      if (in_x) {
+        cpx<R>* o = udst + (size_t)t * W;
 #pragma unroll
-          for (int m = 0; m < N2; ++m) colB[(t + N1 * m) * RS] = v[m] * sc;
+        for (int m = 0; m < N1; ++m) {
+          *o = u[m];
+          o += N2 * W;
         }
       }
-      __syncthreads();
-      cpx<R>* udst = U + (size_t)jj * g.NI * C * H * W + ((size_t)img * C + lcc) * H * W + x0 + lxc;
-      if (lin)
-        for (int y = threadIdx.x / CT; y < H; y += ystep) udst[(size_t)y * W] = tileB[y * RS + lc];
     }
+    __syncthreads();  // the exchange is read before the next window row writes it
   }
 }
 
@@ -618,26 +622,25 @@ cudaError_t row_reg_launch(int C, bool real, int band, const RegLaunch& L, const
   return cudaErrorNotSupported;
 }
 
-template <int N1, int N2, int BAND>
+template <int N, int BAND>
 cudaError_t col_reg_variant(const RegLaunch& L, const ColParams& p, const Grid& g, const void* in, void* out) {
-  auto kern = k_layer_col_reg<float, N1, N2, BAND>;
+  auto kern = k_layer_col_reg<float, N, BAND>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
   if (e != cudaSuccess) return e;
   kern<<<L.grid, L.threads, L.smem, L.st>>>(p, g, (const cpx<float>*)in, (cpx<float>*)out);
   return cudaGetLastError();
 }
 
-// band variants (row_band_pick of the H axis) for the diagonal operator of
-// sides with N2 % N1 == 0; the caller passes band 0 for any other operator
-template <int N1, int N2>
+// band variants (col_band_pick of the H axis) for the diagonal operator between
+// a forward and an inverse transform; the caller passes band 0 otherwise
+template <int N>
 cudaError_t col_reg_launch(int band, const RegLaunch& L, const ColParams& p, const Grid& g, const void* in, void* out) {
-  if constexpr (N2 % N1 == 0) {
-    if constexpr (row_band_ok(N2, 1))
-      if (band == 1) return col_reg_variant<N1, N2, 1>(L, p, g, in, out);
-    if constexpr (row_band_ok(N2, 2))
-      if (band == 2) return col_reg_variant<N1, N2, 2>(L, p, g, in, out);
-  }
-  return col_reg_variant<N1, N2, 0>(L, p, g, in, out);
+  constexpr int n2 = N / col_n1(N);
+  if constexpr (row_band_ok(n2, 1))
+    if (band == 1) return col_reg_variant<N, 1>(L, p, g, in, out);
+  if constexpr (row_band_ok(n2, 2))
+    if (band == 2) return col_reg_variant<N, 2>(L, p, g, in, out);
+  return col_reg_variant<N, 0>(L, p, g, in, out);
 }
 
 template <int N1, int N2>
@@ -670,7 +673,7 @@ cudaError_t fft_rows_reg_launch(bool inv, const RegLaunch& L, const void* src, v
   }                                                                                                            \
   cudaError_t col_reg_##N(int band, const RegLaunch& L, const ColParams& p, const Grid& g, const void* in,       \
                           void* out) {                                                                         \
-    return col_reg_launch<reg_lanes(N), N / reg_lanes(N)>(band, L, p, g, in, out);                             \
+    return col_reg_launch<N>(band, L, p, g, in, out);                             \
   }                                                                                                            \
   cudaError_t fft_rows_reg_##N(bool inv, const RegLaunch& L, const void* src, void* dst, int nlines, const void* tw, \
                                float scale) {                                                                  \

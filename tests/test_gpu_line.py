@@ -58,3 +58,56 @@ def test_line_passes_not_finite(spoil):
     assert not np.isfinite(a[0, 1]).any() and not np.isfinite(b[0, 1]).any()
     for i in ((0, 0), (1, 0), (1, 1)):
         assert np.linalg.norm(a[i] - b[i]) <= 2e-14 * np.linalg.norm(b[i])
+
+
+REG_SIDES = (64, 80, 96, 112, 128, 144, 160, 192, 224, 240, 256, 288, 320, 336, 384, 400, 432, 448, 480, 512, 1024)
+
+
+def _mixed(shape, method, diffraction, schedule, pixelsize):
+    import torch
+
+    from dtmm_gb300 import samples
+    from dtmm_gb300.illumination import illumination_device
+    from dtmm_gb300.transfer import plan_transfer
+
+    wl = [450.0, 620.0]
+    mat = samples.twisted_nematic_device(shape, 2, no=1.52, ne=1.71, amplitude=0.3, seed=6)
+    fin = illumination_device(shape, wl, pixelsize, beta=0.1, phi=0.4, precision="mixed")
+    plan = plan_transfer(tuple(fin.shape), wl, pixelsize, mat, beta=0.1, phi=0.4, method=method,
+                         diffraction=diffraction, npass=1, precision="mixed", tuning=dict(fft_schedule=schedule))
+    out = torch.full_like(fin, float("nan"))
+    plan.workspace.fill_(255)  # unwritten columns hold NaN
+    plan.run(fin, out)
+    return out.cpu().numpy()
+
+
+@pytest.mark.parametrize("height", REG_SIDES)
+@pytest.mark.parametrize("method,diffraction,pixelsize", [("4x4", 3, 50.0), ("2x2", 1, 100.0), ("4x4", 1, 220.0)])
+def test_register_columns_match_shared_memory_passes(height, method, diffraction, pixelsize):
+    """complex64 column pass of every register side, narrow band, wider band and (220 nm pixels) no band
+    limit; the workspace starts as NaN, so nothing beyond the band may be read.  Eight transforms of
+    relative error below 3e-7 on either side, at random: 3e-6."""
+    shape = (height, 80 if height != 80 else 64)
+    a = _mixed(shape, method, diffraction, 0, pixelsize)
+    b = _mixed(shape, method, diffraction, 2, pixelsize)
+    assert np.linalg.norm(a - b) <= 3e-6 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("shape", [(64, 50), (150, 96)])
+def test_line_passes_read_no_column_beyond_the_band(shape):
+    import torch
+
+    from dtmm_gb300 import samples
+    from dtmm_gb300.illumination import illumination_device
+    from dtmm_gb300.transfer import plan_transfer
+
+    wl = [450.0, 620.0]
+    mat = samples.twisted_nematic_device(shape, 2, no=1.52, ne=1.71, amplitude=0.3, seed=6)
+    fin = illumination_device(shape, wl, 50.0, precision="double")
+    plan = plan_transfer(tuple(fin.shape), wl, 50.0, mat, method="4x4", diffraction=3, npass=1, precision="double")
+    out = torch.empty_like(fin)
+    plan.run(fin, out)
+    again = torch.empty_like(fin)
+    plan.workspace.fill_(255)
+    plan.run(fin, again)
+    assert torch.equal(out, again)
