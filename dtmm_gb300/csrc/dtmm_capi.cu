@@ -770,8 +770,14 @@ struct Engine {
     } else {
       const int n1 = reg_lanes(d.width);
       const int nl = p.G * p.PB * C;
-      const size_t smem =
-          2 * (size_t)nl * reg_row_stride(n1, d.width) * sizeof(cpx<R>) + d.width * sizeof(cpx<R>);
+      RowParams q = p;
+      // several windows, as many lines a block as the variant takes: accumulators
+      // in registers; one window: in place
+      q.xr = re && xr_pixels(d.width) > 0 && nl == kXrLines && p.PB <= 2 && d.nlam % p.G == 0 && d.npol % p.PB == 0
+                 ? 1 : 0;
+      if (re && (L.nwin == 1 || p.win_only >= 0)) q.xr = -1;
+      const size_t smem = (q.xr != 0 ? 1 : 2) * (size_t)nl * reg_row_stride(n1, d.width) * sizeof(cpx<R>) +
+                          d.width * sizeof(cpx<R>);
       if (smem > 220 * 1024 || nl * n1 > reg_row_max_threads(d.width))
         return fail(DTMM_ENOTSUP, "row of %d pixels too large for one block", d.width);
       RegLaunch rl;
@@ -782,11 +788,7 @@ struct Engine {
       // one layer's operator records beyond half of L2 (128 MB): the groups of
       // a row run next to each other and share the row's records in L2
       const size_t rec_bytes = (re ? sizeof(R) : sizeof(cpx<R>)) * (size_t)d.nray * L.nwin * p.rec_stride * L.HW;
-      RowParams q = p;
       q.groups_inner = rec_bytes > ((size_t)64 << 20) ? 1 : 0;
-      // 256-point rows of the 4x4 method, two images a block in every block:
-      // accumulators in registers, two pixels a thread
-      q.xr = (C == 4 && re && d.width == 256 && nl == kXrLines && d.nlam % p.G == 0 && d.npol % p.PB == 0) ? 2 : 0;
       rl.grid = q.groups_inner ? dim3(d.nray * ngrp * npg, d.height) : dim3(d.height, d.nray * ngrp * npg);
       rl.st = st;
       mark(PROF_ROW);
@@ -1908,7 +1910,8 @@ struct Engine {
   }
 
   // byte offset of the backward-mode records in a voxel's operator records
-  size_t back_records() const { return (size_t)REC_BLOCK * (real_ops() ? sizeof(R) : sizeof(cpx<R>)); }
+  // the backward blocks' planes of a row of records
+  size_t back_records() const { return (size_t)REC_BLOCK * d.width * (real_ops() ? sizeof(R) : sizeof(cpx<R>)); }
 
   // 2x2 method in k-space (reflection 0 or 1; dtmm/propagate_2x2.py:19-87,
   // :193-284 driven by dtmm/transfer.py:1074-1183) over npass passes that

@@ -146,7 +146,7 @@ struct OpParams {
   double scale;          // folded into the records (the row pass's inverse-transform scale)
 };
 
-// Records per voxel and window, [ray][window][H][W][record] (REC_BLOCK per
+// Records per voxel and window, [ray][window][H][record pair][W][2] (REC_BLOCK per
 // mode block): complex, or real when the host has proven the real path (real
 // eps above beta^2 everywhere).
 
@@ -285,7 +285,8 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
   ff e0 = z, e2 = z, n0 = z;
   float caf = 0.0f, saf = 0.0f, ctf = 0.0f, scaf = 0.0f, ssaf = 0.0f, ief = 0.0f;  // FP32 copies for E
   bool iso = false;
-  size_t slot = 0;
+  size_t row = 0;
+  int xs = 0;
   const ff dd = ff_of(p.d);
   if (active) {
     const int y = pix / g.W, x = pix - y * g.W;
@@ -306,7 +307,8 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
     scaf = ff_f(ff_mul(vx.st, vx.ca));
     ssaf = ff_f(ff_mul(vx.st, vx.sa));
     ief = ff_f(ff_div(ff_mk(1.0f, 0.0f), e0));
-    slot = (size_t)y * g.W + (p.permW ? p.permW[x] : x);
+    row = (size_t)y * g.W;
+    xs = p.permW ? p.permW[x] : x;
   }
   const int rw0 = ray0 * p.nwin, rw1 = ray1 * p.nwin;
   for (int c0 = rw0; c0 < rw1; c0 += kLeanChunk) {
@@ -411,7 +413,7 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
           rec[11] = -r6;
         }
       }
-      store_recs<nrec, float>(opv + ((size_t)(c0 + k) * HW + slot) * nrec, rec);
+      store_planes<nrec, float>(opv + ((size_t)(c0 + k) * HW + row) * nrec, g.W, xs, rec);
     }
   }
 }
@@ -436,7 +438,8 @@ __global__ void k_voxel_op(OpParams p, Grid g, void* __restrict__ opv) {
   const double theta = p.epsa[ao + 1], azim = p.epsa[ao + 2];
   if (p.eps_dev != nullptr) p.eps_eff = mk<double>(p.eps_dev[0], p.eps_dev[1]);
   constexpr int nrec = FOUR ? OP_REC : REC_BLOCK;
-  const size_t slot = (size_t)y * g.W + (p.permW ? p.permW[x] : x);
+  const size_t row = (size_t)y * g.W;
+  const int xs = p.permW ? p.permW[x] : x;
   // the voxel's trigonometry and invariants, shared by every ray and window
   double sa, ca;
   sincos(azim, &sa, &ca);
@@ -490,7 +493,7 @@ __global__ void k_voxel_op(OpParams p, Grid g, void* __restrict__ opv) {
           rec[11] = to_r<R>((al[3] + aw) * p.d);
         }
       }
-      store_recs<nrec, R>((R*)opv + ((size_t)rw * HW + slot) * nrec, rec);
+      store_planes<nrec, R>((R*)opv + ((size_t)rw * HW + row) * nrec, g.W, xs, rec);
     }
     return;
   }
@@ -611,7 +614,7 @@ __global__ void k_voxel_op(OpParams p, Grid g, void* __restrict__ opv) {
       rec[11] = cvt<R>((al[3] + aw) * p.d);
     }
   }
-  store_recs<nrec, cpx<R>>((cpx<R>*)opv + ((size_t)rw * HW + slot) * nrec, rec);
+  store_planes<nrec, cpx<R>>((cpx<R>*)opv + ((size_t)rw * HW + row) * nrec, g.W, xs, rec);
   }
 }
 
@@ -2412,7 +2415,7 @@ __global__ void __launch_bounds__(256, 3) k_layer_row(RowParams p, Grid g, const
       constexpr int NR = C == 4 ? OP_REC : REC_BLOCK;
       for (int q = threadIdx.x; q < W; q += blockDim.x) {
         T rec[NR];
-        load_recs<NR, T>(opw + (size_t)q * rs, rec);
+        load_planes<NR, T>(opw, W, q, rec);
         const T* ef = rec;
         const T* eb = rec + (C == 4 ? REC_BLOCK : 0);
         for (int gl = 0; gl < G; ++gl) {

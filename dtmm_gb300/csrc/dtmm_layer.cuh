@@ -7,7 +7,7 @@
 //                          image = (ray * npol + pol) * nlam + lam
 //                          (the reference's ([rays],[pols],lambda,4,H,W) order)
 //   window-row buffers   : [j][image][component][H][W]
-//   layer operators      : [ray][window][H][W][record], 6 records per mode
+//   layer operators      : [ray][window][H][record pair][W][2], 6 records per mode
 //                          block (forward, then backward with both blocks)
 #pragma once
 
@@ -20,8 +20,10 @@ namespace dtmm {
 // column scaled by the scale of the pass over det(E), and the two phase
 // arguments, (e0 s, e1, e2 s, e3, arg0, arg1) with s = scale / det(E).
 // E' = E diag(s, 1) has det(E') = scale, so E' diag(p) adj(E') = scale E
-// diag(p) E^-1.  A voxel keeps its records next to each other (REC_BLOCK
-// or 2 REC_BLOCK of them), so they are read with vector loads.
+// diag(p) E^-1.  A row of voxels keeps them as planes of record pairs, [row]
+// [pair][x][2]: consecutive voxels read and write consecutive 8 (16) bytes.  (A
+// voxel's twelve FP32 records next to each other cost the L1 pipe three times
+// the wavefronts, a fifth of the row pass's for 320-point rows and one window.)
 constexpr int REC_BLOCK = 6;
 constexpr int OP_REC = 2 * REC_BLOCK;  // records of both blocks
 
@@ -107,7 +109,7 @@ struct RowParams {
   int nx, ny;            // windows per axis (1, 1 without windows)
   const void* cx;        // [ray][i][lam][W] (null = weight 1)
   const int* wzero;      // [ray][nx*ny]
-  const void* op;        // [ray][win][H][W][rec_stride] (offset to the block the pass uses)
+  const void* op;        // [ray][win][H][rec_stride / 2][W][2] (offset to the block the pass uses)
   int rec_stride;        // records per voxel: REC_BLOCK, or OP_REC with both blocks
   const double* ks;      // [lam]
   double dir;            // propagation direction (+1 / -1)
@@ -122,7 +124,8 @@ struct RowParams {
   int accumulate;        // add the result to X instead of overwriting it
   int band_out;          // 1: columns beyond the band need not be written (ColParams::xband reads them as zeros)
   int groups_inner;      // register row pass: blockIdx.x the group, blockIdx.y the row (else the reverse)
-  int xr;                // register row pass variant with accumulators in registers, pixels a thread (0: none)
+  int xr;                // register row pass variant: -1 one window in place, 1 accumulators in registers,
+                         // 0 accumulators in shared memory
 };
 
 template <typename R>
@@ -204,6 +207,33 @@ __device__ __forceinline__ void store_recs(T* __restrict__ dst, const T (&r)[N])
   }
 }
 
+// r a + c, real r
+__device__ __forceinline__ cpx<float> rfma(float r, cpx<float> a, cpx<float> c) {
+  const float2 v = __ffma2_rn(make_float2(a.re, a.im), make_float2(r, r), make_float2(c.re, c.im));
+  return mk<float>(v.x, v.y);
+}
+
+// the first N operator records of pixel x of a row: planes of record pairs
+// (see REC_BLOCK)
+template <int N, typename T>
+__device__ __forceinline__ void load_planes(const T* __restrict__ row, int W, int x, T (&r)[N]) {
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    T two[2];
+    load_recs<2, T>(row + ((size_t)i * W + x) * 2, two);
+    r[2 * i] = two[0];
+    r[2 * i + 1] = two[1];
+  }
+}
+template <int N, typename T>
+__device__ __forceinline__ void store_planes(T* __restrict__ row, int W, int x, const T (&r)[N]) {
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    const T two[2] = {r[2 * i], r[2 * i + 1]};
+    store_recs<2, T>(row + ((size_t)i * W + x) * 2, two);
+  }
+}
+
 // one 2x2 block of the per-voxel operator, out += E' diag(p0, p1) adj(E') h
 // (E' the block's records, first column carrying scale / det, so det(E') =
 // scale), in projector form: with c0 = (e0', e2') and r0 = (e3, -e1),
@@ -212,9 +242,15 @@ __device__ __forceinline__ void store_recs(T* __restrict__ dst, const T (&r)[N])
 template <typename R, typename T>
 __device__ __forceinline__ void apply_block(const T e[4], cpx<R> q, cpx<R> dp, cpx<R> h0, cpx<R> h1, cpx<R>& a0,
                                             cpx<R>& a1) {
-  const cpx<R> s = (e[3] * h0 - e[1] * h1) * dp;
-  a0 = cfma(q, h0, a0) + e[0] * s;
-  a1 = cfma(q, h1, a1) + e[2] * s;
+  if constexpr (sizeof(R) == 4 && sizeof(T) == 4) {
+    const cpx<R> s = rfma(-e[1], h1, e[3] * h0) * dp;
+    a0 = rfma(e[0], s, cfma(q, h0, a0));
+    a1 = rfma(e[2], s, cfma(q, h1, a1));
+  } else {
+    const cpx<R> s = (e[3] * h0 - e[1] * h1) * dp;
+    a0 = cfma(q, h0, a0) + e[0] * s;
+    a1 = cfma(q, h1, a1) + e[2] * s;
+  }
 }
 
 }  // namespace dtmm

@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
     constexpr int NR = C == 4 ? OP_REC : REC_BLOCK;
     for (int x = threadIdx.x; x < W; x += blockDim.x) {
       T rec[NR];
-      load_recs<NR, T>(opw + (size_t)x * rs, rec);
+      load_planes<NR, T>(opw, W, x, rec);
       const int xm = (int)((x * rcp2) >> 16), q = slot(x - xm * n2, xm);
       const T* ef = rec;
       const T* eb = rec + (C == 4 ? REC_BLOCK : 0);

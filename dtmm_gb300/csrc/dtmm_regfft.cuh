@@ -143,11 +143,11 @@ struct SmallDFT {
       v[1] = a - b;
     } else if constexpr (P == 4) {
       const cpx<R> s02 = v[0] + v[2], d02 = v[0] - v[2], s13 = v[1] + v[3], d13 = v[1] - v[3];
-      const cpx<R> jd = INV ? mk<R>(-d13.im, d13.re) : mk<R>(d13.im, -d13.re);
       v[0] = s02 + s13;
       v[2] = s02 - s13;
-      v[1] = d02 + jd;
-      v[3] = d02 - jd;
+      // d02 -+ i d13: the components cross, so they are summed one by one
+      v[INV ? 1 : 3] = mk<R>(d02.re - d13.im, d02.im + d13.re);
+      v[INV ? 3 : 1] = mk<R>(d02.re + d13.im, d02.im - d13.re);
     } else {
       cpx<R> x[P];
 #pragma unroll

@@ -69,20 +69,36 @@ __host__ __device__ constexpr int row_band_pick(int n, int lim) {
   return 0;
 }
 
-// Launch bounds: rows of up to 16 points per lane run at most 256 threads a
-// block and keep at most 85 registers, so that six 128-thread blocks share an
-// SM (measured 8 % faster than four at 117 registers for 256-point rows);
-// 32 points per lane need the registers of a whole 512-thread block.
-// XR > 0: the block holds exactly kXrLines lines (two images of the 4x4
-// method) and W / XR threads, and each thread keeps the accumulators of its
-// XR pixels in registers across the windows (no shared-memory
-// read-modify-write per window); 128 registers a thread at most.
+// Launch bounds: rows of up to 16 points per lane, and single-window rows, keep
+// at most 80 registers, so that six 128-thread blocks share an SM (measured 8 %
+// faster than four at 117 registers for 256-point rows); with several windows
+// and more than 16 points per lane the spills of that cost more than the warps
+// (320 points, nine windows: 244 us a layer, 221 with 128 registers); 32 points
+// per lane need the registers of a whole 512-thread block.
+// XR > 0 (several windows, 16 points a lane): the block holds kXrLines lines and
+// W / XR threads, and each thread keeps the accumulators of its XR pixels in
+// registers across the windows: no second set of lines and no shared-memory
+// read-modify-write per window (nine windows, one layer: 128 points 40 -> 31 us,
+// 256 points of the 2x2 method 66 -> 48 us).
+// XR = -1: one window (no windows, or a single-window chain).  There is nothing
+// to accumulate: the operators' results replace the transformed rows in place,
+// without the second set of lines (half the shared memory, so twice the blocks
+// a SM) and its clearing, reads and writes.  320 points, 70
+// images: 166 -> 146 us a layer.
 constexpr int kXrLines = 8;
+// pixels a thread of that variant (0: the side has none): 16 points a lane, 128
+// registers a thread with the accumulators; with 32 points a lane (168 registers)
+// it took 1.35 ms a layer for 1024-point rows against 1.27 ms in shared memory
+__host__ __device__ constexpr int xr_pixels(int n) {
+  const int n1 = reg_lanes(n);
+  return n1 > 0 && n == 16 * n1 ? n / (kXrLines * n1) : 0;
+}
 template <typename R, int C, bool REAL, int N1, int N2, int BAND, int XR = 0>
 __global__ void __launch_bounds__(XR > 0 ? (N1 * N2) / (XR > 0 ? XR : 1) : (N2 >= 32 ? 512 : 256),
-                                  XR > 0 ? 4 : (N2 >= 32 ? 1 : 3))
+                                  XR > 0 ? 512 / (kXrLines * N1) : (N2 >= 32 ? 1 : (XR == 0 && N2 > 16 ? 2 : 3)))
     k_layer_row_reg(RowParams p, Grid g, const cpx<R>* __restrict__ U, cpx<R>* __restrict__ X) {
-  static_assert(XR == 0 || C == 4, "register accumulators: the 4x4 method's two-image blocks");
+  constexpr bool ONE = XR < 0;
+  constexpr int XL = kXrLines;
   using T = typename std::conditional<REAL, R, cpx<R>>::type;
   using TS = TwoStep<N1, N2>;
   constexpr int W = N1 * N2;
@@ -103,19 +119,19 @@ __global__ void __launch_bounds__(XR > 0 ? (N1 * N2) / (XR > 0 ? XR : 1) : (N2 >
   const int NP = min(p.PB, g.npol - pol0);  // polarisations of this block
   const int nlines = G * NP * C;
   cpx<R>* acc = (cpx<R>*)smem_raw;                  // [lines][LS]
-  cpx<R>* tmp = acc + (size_t)p.G * p.PB * C * LS;  // [lines][LS] exchange and transformed rows
+  cpx<R>* tmp = acc + (XR != 0 ? 0 : (size_t)p.G * p.PB * C * LS);  // [lines][LS] exchange and transformed rows
   cpx<R>* tw = tmp + (size_t)p.G * p.PB * C * LS;   // [W]  twiddles, lane-major (TwoStep::twiddle_entry)
   const int HW = H * W;
   const int nwin = p.nx * p.ny;
   for (int e = threadIdx.x; e < W; e += blockDim.x) tw[e] = TS::twiddle_entry((const cpx<R>*)p.tw, e);
   if (XR == 0)
     for (int e = threadIdx.x; e < nlines * LS; e += blockDim.x) acc[e] = mk<R>(0, 0);
-  cpx<R> racc[XR > 0 ? XR : 1][kXrLines];
+  cpx<R> racc[XR > 0 ? XR : 1][XL];
   if (XR > 0) {
 #pragma unroll
     for (int k = 0; k < (XR > 0 ? XR : 1); ++k)
 #pragma unroll
-      for (int l = 0; l < kXrLines; ++l) racc[k][l] = mk<R>((R)0, (R)0);
+      for (int l = 0; l < XL; ++l) racc[k][l] = mk<R>((R)0, (R)0);
   }
   // phase scale k0 * direction of each wavelength of the block (formed once, in FP64)
   __shared__ R s_kph[kMaxRowGroup];
@@ -182,30 +198,36 @@ __global__ void __launch_bounds__(XR > 0 ? (N1 * N2) / (XR > 0 ? XR : 1) : (N2 >
       constexpr int XU = (C == 2 && N2 >= 32) ? 4 : 1;
       constexpr int NR = C == 4 ? OP_REC : REC_BLOCK;  // records this pass reads per voxel
       if constexpr (XR > 0) {
-        // pixels threadIdx.x + k W / XR; the block's two images b (G = 1 and
-        // two polarisations share the phases, G = 2 has its own per image)
+        // pixels threadIdx.x + k W / XR of the block's images b (full blocks of one
+        // or two polarisations, which share their wavelength's phases)
 #pragma unroll
         for (int k = 0; k < (XR > 0 ? XR : 1); ++k) {
           const int x = threadIdx.x + k * (W / (XR > 0 ? XR : 1));
           T rec[NR];
-          load_recs<NR, T>(opw + (size_t)x * rs, rec);
+          load_planes<NR, T>(opw, W, x, rec);
           const T* ef = rec;
-          const T* eb = rec + REC_BLOCK;
+          const T* eb = rec + (C == 4 ? REC_BLOCK : 0);
           cpx<R> qf, dpf, qb, dpb;
 #pragma unroll
-          for (int b = 0; b < 2; ++b) {
-            if (b == 0 || G == 2) {
-              const R kph = s_kph[G == 2 ? b : 0];
+          for (int b = 0; b < XL / C; ++b) {
+            if (b % 2 == 0 || NP == 1) {
+              const R kph = s_kph[NP == 1 ? b : b / 2];
               const cpx<R> f0 = phase_of(ef[4], kph), f1 = phase_of(ef[5], kph);
               qf = f1 * sc;
               dpf = f0 - f1;
-              const cpx<R> b0 = phase_of(eb[4], kph), b1 = phase_of(eb[5], kph);
-              qb = b1 * sc;
-              dpb = b0 - b1;
+              if (C == 4) {
+                const cpx<R> b0 = phase_of(eb[4], kph), b1 = phase_of(eb[5], kph);
+                qb = b1 * sc;
+                dpb = b0 - b1;
+              }
             }
-            const cpx<R>* h = tmp + (size_t)(4 * b) * LS + x;
-            apply_block<R, T>(ef, qf, dpf, h[0], h[2 * LS], racc[k][4 * b], racc[k][4 * b + 2]);
-            apply_block<R, T>(eb, qb, dpb, h[LS], h[3 * LS], racc[k][4 * b + 1], racc[k][4 * b + 3]);
+            const cpx<R>* h = tmp + (size_t)(C * b) * LS + x;
+            if (C == 4) {
+              apply_block<R, T>(ef, qf, dpf, h[0], h[2 * LS], racc[k][C * b], racc[k][C * b + 2 % C]);
+              apply_block<R, T>(eb, qb, dpb, h[LS], h[3 * LS], racc[k][C * b + 1], racc[k][C * b + 3 % C]);
+            } else {
+              apply_block<R, T>(ef, qf, dpf, h[0], h[LS], racc[k][C * b], racc[k][C * b + 1]);
+            }
           }
         }
         __syncthreads();
@@ -217,7 +239,7 @@ __global__ void __launch_bounds__(XR > 0 ? (N1 * N2) / (XR > 0 ? XR : 1) : (N2 >
         for (int k = 0; k < XU; ++k) {
           const int x = x0 + k * blockDim.x;
           if (x >= W) break;
-          load_recs<NR, T>(opw + (size_t)x * rs, rec[k]);
+          load_planes<NR, T>(opw, W, x, rec[k]);
         }
 #pragma unroll
         for (int k = 0; k < XU; ++k) {
@@ -243,7 +265,18 @@ __global__ void __launch_bounds__(XR > 0 ? (N1 * N2) / (XR > 0 ? XR : 1) : (N2 >
               const int l0 = (g2 * NP + q) * C;
               const cpx<R>* h = tmp + (size_t)l0 * LS + x;
               cpx<R>* a = acc + (size_t)l0 * LS + x;
-              if (C == 4) {
+              if constexpr (ONE) {
+                const cpx<R> z = mk<R>((R)0, (R)0);
+                cpx<R> a0 = z, a1 = z, a2 = z, a3 = z;
+                if (C == 4) {
+                  apply_block<R, T>(ef, qf, dpf, h[0], h[2 * LS], a0, a2);
+                  apply_block<R, T>(eb, qb, dpb, h[LS], h[3 * LS], a1, a3);
+                  a[0] = a0; a[LS] = a1; a[2 * LS] = a2; a[3 * LS] = a3;
+                } else {
+                  apply_block<R, T>(ef, qf, dpf, h[0], h[LS], a0, a1);
+                  a[0] = a0; a[LS] = a1;
+                }
+              } else if (C == 4) {
                 cpx<R> a0 = a[0], a1 = a[LS], a2 = a[2 * LS], a3 = a[3 * LS];
                 apply_block<R, T>(ef, qf, dpf, h[0], h[2 * LS], a0, a2);
                 apply_block<R, T>(eb, qb, dpb, h[LS], h[3 * LS], a1, a3);
@@ -264,7 +297,7 @@ __global__ void __launch_bounds__(XR > 0 ? (N1 * N2) / (XR > 0 ? XR : 1) : (N2 >
 #pragma unroll
     for (int k = 0; k < (XR > 0 ? XR : 1); ++k)
 #pragma unroll
-      for (int l = 0; l < kXrLines; ++l) acc[(size_t)l * LS + threadIdx.x + k * (W / (XR > 0 ? XR : 1))] = racc[k][l];
+      for (int l = 0; l < XL; ++l) acc[(size_t)l * LS + threadIdx.x + k * (W / (XR > 0 ? XR : 1))] = racc[k][l];
     __syncthreads();
   }
   if (active) {
@@ -272,6 +305,7 @@ __global__ void __launch_bounds__(XR > 0 ? (N1 * N2) / (XR > 0 ? XR : 1) : (N2 >
     const cpx<R>* al = acc + (size_t)line * LS;
 #pragma unroll
     for (int m = 0; m < N2; ++m) v[m] = al[t + N1 * m];
+    if (XR != 0) __syncwarp(gm);  // the line is read before the exchange overwrites it
     TS::template step1<R, false>(v, xl, 1, TWREG ? trow : nullptr, tw, t);
     __syncwarp(gm);
     cpx<R> u[TS::J][N1];
@@ -287,14 +321,19 @@ __global__ void __launch_bounds__(XR > 0 ? (N1 * N2) / (XR > 0 ? XR : 1) : (N2 >
         dst[t + N1 * m] = p.accumulate ? dst[t + N1 * m] + v[m] : v[m];
       }
     } else {
-      __syncwarp(gm);
-      TS::template store<R>(u, xl, 1, t, (R)1);
-      __syncwarp(gm);
+      // straight from the second step's registers: N1 (or the last round's
+      // N2 % N1) consecutive points a store
 #pragma unroll
-      for (int m = 0; m < N2; ++m) {
-        if (BAND != 0 && m >= KBO && m < N2 - KBO && p.band_out) continue;
-        const cpx<R> r = xl[t + N1 * m];
-        dst[t + N1 * m] = p.accumulate ? dst[t + N1 * m] + r : r;
+      for (int j = 0; j < TS::J; ++j) {
+        const int k1 = t + N1 * j;
+        if (k1 < N2) {
+#pragma unroll
+          for (int k2 = 0; k2 < N1; ++k2) {
+            const int e = k1 + N2 * k2;
+            if (BAND != 0 && e >= KBO * N1 && e < W - KBO * N1 && p.band_out) continue;
+            dst[e] = p.accumulate ? dst[e] + u[j][k2] : u[j][k2];
+          }
+        }
       }
     }
   }
@@ -591,16 +630,23 @@ cudaError_t row_reg_variant(const RegLaunch& L, const RowParams& p, const Grid& 
 }
 
 // real records with a band variant b (row_band_pick), every (C, REAL) dense
-// (p.xr > 0: the register-accumulator variant, built for 256-point rows of
-// the 4x4 method, XR = p.xr pixels a thread)
+// (p.xr: the variant, RowParams)
 template <int N1, int N2, int C>
 cudaError_t row_reg_real(int band, const RegLaunch& L, const RowParams& p, const Grid& g, const void* U, void* X) {
-  if constexpr (N1 == 16 && N2 == 16 && C == 4) {
-    if (p.xr == 2) {
-      if (band == 1) return row_reg_variant<N1, N2, C, true, 1, 2>(L, p, g, U, X);
-      if (band == 2) return row_reg_variant<N1, N2, C, true, 2, 2>(L, p, g, U, X);
-      return row_reg_variant<N1, N2, C, true, 0, 2>(L, p, g, U, X);
+  if constexpr (xr_pixels(N1 * N2) > 0) {
+    constexpr int XR = xr_pixels(N1 * N2);
+    if (p.xr > 0) {
+      if (band == 1) return row_reg_variant<N1, N2, C, true, 1, XR>(L, p, g, U, X);
+      if (band == 2) return row_reg_variant<N1, N2, C, true, 2, XR>(L, p, g, U, X);
+      return row_reg_variant<N1, N2, C, true, 0, XR>(L, p, g, U, X);
     }
+  }
+  if (p.xr < 0) {
+    if constexpr (row_band_ok(N2, 1))
+      if (band == 1) return row_reg_variant<N1, N2, C, true, 1, -1>(L, p, g, U, X);
+    if constexpr (row_band_ok(N2, 2))
+      if (band == 2) return row_reg_variant<N1, N2, C, true, 2, -1>(L, p, g, U, X);
+    return row_reg_variant<N1, N2, C, true, 0, -1>(L, p, g, U, X);
   }
   if constexpr (row_band_ok(N2, 1))
     if (band == 1) return row_reg_variant<N1, N2, C, true, 1>(L, p, g, U, X);
