@@ -25,10 +25,17 @@ template <typename R>
 __host__ __device__ __forceinline__ cpx<R> operator+(cpx<R> a, cpx<R> b) { return mk<R>(a.re + b.re, a.im + b.im); }
 template <typename R>
 __host__ __device__ __forceinline__ cpx<R> operator-(cpx<R> a, cpx<R> b) { return mk<R>(a.re - b.re, a.im - b.im); }
+// f32x2 instructions (the library is built for sm_103a; host tests compile
+// these headers for nvcc's default architecture)
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000
+#define DTMM_F32X2 1
+#else
+#define DTMM_F32X2 0
+#endif
 // complex64 sums as one packed operation (sm_100 f32x2: half the issue slots,
 // the same rounding)
 __host__ __device__ __forceinline__ cpx<float> operator+(cpx<float> a, cpx<float> b) {
-#ifdef __CUDA_ARCH__
+#if DTMM_F32X2
   const float2 r = __fadd2_rn(make_float2(a.re, a.im), make_float2(b.re, b.im));
   return mk<float>(r.x, r.y);
 #else
@@ -36,7 +43,7 @@ __host__ __device__ __forceinline__ cpx<float> operator+(cpx<float> a, cpx<float
 #endif
 }
 __host__ __device__ __forceinline__ cpx<float> operator-(cpx<float> a, cpx<float> b) {
-#ifdef __CUDA_ARCH__
+#if DTMM_F32X2
   const float2 r = __ffma2_rn(make_float2(b.re, b.im), make_float2(-1.0f, -1.0f), make_float2(a.re, a.im));
   return mk<float>(r.x, r.y);
 #else

@@ -209,8 +209,12 @@ __device__ __forceinline__ void store_recs(T* __restrict__ dst, const T (&r)[N])
 
 // r a + c, real r
 __device__ __forceinline__ cpx<float> rfma(float r, cpx<float> a, cpx<float> c) {
+#if DTMM_F32X2
   const float2 v = __ffma2_rn(make_float2(a.re, a.im), make_float2(r, r), make_float2(c.re, c.im));
   return mk<float>(v.x, v.y);
+#else
+  return mk<float>(fmaf(r, a.re, c.re), fmaf(r, a.im, c.im));
+#endif
 }
 
 // the first N operator records of pixel x of a row: planes of record pairs
