@@ -10,9 +10,8 @@ sRGB or gray image (``specter2color``, dtmm/color.py:52-224).  ``pom_image``
 does the three steps in one pass per pixel.
 
 Arrays may be numpy (copied to the device and back) or CUDA tensors (results
-stay on the device).  A caller that enqueues the image behind other work on
-the same stream passes ``pmat`` and ``cmf`` as device tensors: a host-to-device
-copy from pageable memory would wait for that work.  The small jones / 4x4
+stay on the device).  ``pmat`` and ``cmf`` may be device tensors; host ones are
+copied in stream order without waiting for queued work.  The small jones / 4x4
 matrices are built on the host (``jonesvec``, ``polarizer``,
 ``rotated_matrix``, ``ray_jonesmat4x4``).
 Refocusing goes through a per-k diffraction matrix (``diffract``, the
@@ -154,6 +153,12 @@ def _dev_field(field):
     return torch.from_numpy(np.ascontiguousarray(a, dtype)).cuda(), True
 
 
+def _upload(a, device):
+    """A small host array on the device, in stream order: the copy is staged before the call returns, and
+    the work queued before it is not waited for."""
+    return _torch().from_numpy(np.ascontiguousarray(a)).to(device, non_blocking=True)
+
+
 def _dev_real(x, device):
     torch = _torch()
     if x is None:
@@ -199,7 +204,7 @@ def _desc(f, jvec, pmat, window):
         if isinstance(pmat, torch.Tensor):  # already on the device: no upload behind queued work
             pt = pmat.to(device=f.device, dtype=torch.complex128).contiguous()
         else:
-            pt = torch.from_numpy(np.ascontiguousarray(np.asarray(pmat, np.complex128))).to(f.device)
+            pt = _upload(np.asarray(pmat, np.complex128), f.device)
         if tuple(pt.shape) != (4, 4):
             raise NotImplementedError("one 4x4 analyzer matrix for every pixel and wavelength")
         keep.append(pt)
@@ -390,7 +395,7 @@ def pom_image(field, cmf, jvec=None, pmat=None, window=None, norm=False, gamma=T
     if isinstance(cmf, torch.Tensor):  # already on the device: no upload behind queued work
         c = cmf.to(device=f.device, dtype=torch.float64).contiguous()
     else:
-        c = torch.from_numpy(np.ascontiguousarray(np.asarray(cmf, np.float64))).to(f.device)
+        c = _upload(np.asarray(cmf, np.float64), f.device)
     if tuple(c.shape) != (f.shape[-4], 3):
         raise ValueError("cmf must have one row per wavelength")
     rgb = torch.empty(tuple(f.shape[-2:]) + (3,), dtype=torch.float32, device=f.device)
