@@ -78,6 +78,7 @@ size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 constexpr int kPartBlocks = 1216;  // blocks of the effective-medium reduction
 constexpr int kWinChunks = 64;     // blocks per window of the window statistics
+constexpr long long kOpWave = 152 * 16;  // blocks of the voxel operator kernel on the GPU at once
 
 // Workspace layout (byte offsets), shared by the size query and the call.
 struct Layout {
@@ -85,6 +86,7 @@ struct Layout {
   int ny, nx, nwin;
   int nlay_sub; // total sub-steps
   bool cache_ops;
+  bool all_ops;   // cache_ops of one pass, filled by one launch
   size_t cplx;  // bytes of one complex
   size_t HW;
   size_t small, part, twH, permH, twW, permW, cx, cy;
@@ -335,7 +337,13 @@ Layout layout_of(const dtmm_transfer_desc* d) {
   // the real-space and modal paths keep no operator records
   L.op_one = (real_space || real2 || d->diffraction == DTMM_DIFFRACTION_FULL) ? 0 : L.cplx * nrw * OP_REC * L.HW;
   const size_t limit = d->op_cache_bytes ? d->op_cache_bytes : ((size_t)48 << 30);
-  L.cache_ops = passes && L.op_one * (size_t)d->nlayers <= limit;
+  // one pass over a small stack: the operators of every layer in one launch
+  // (voxel_ops; its blocks are one wave of the GPU)
+  L.all_ops = !passes && L.op_one > 0 && d->nlayers > 1 && L.op_one * (size_t)d->nlayers <= std::min(limit, (size_t)32 << 20) &&
+              (long long)((L.HW + 127) / 128) * d->nray * d->nlayers <= kOpWave && nblocks(d) == 1;
+  for (int l = 1; l < d->nlayers && L.all_ops; ++l)
+    L.all_ops = d->thickness[l] / d->nstep[l] == d->thickness[0] / d->nstep[0];
+  L.cache_ops = L.all_ops || (passes && L.op_one * (size_t)d->nlayers <= limit);
   // per-layer cache, or two buffers that alternate between the layer being
   // swept and the next layer's operators computed beside it
   L.op = take(L.op_one * (L.cache_ops ? (size_t)d->nlayers : 2));
@@ -1000,7 +1008,7 @@ struct Engine {
     return w;
   }
 
-  int voxel_ops(int layer, double dsub, cpx<R>* op, cudaStream_t s = nullptr) {
+  int voxel_ops(int layer, double dsub, cpx<R>* op, cudaStream_t s = nullptr, int layers = 1) {
     if (s == nullptr) s = st;
     OpParams p;
     memset(&p, 0, sizeof(p));
@@ -1014,6 +1022,7 @@ struct Engine {
     }
     p.eps_complex = d.eps_complex;
     p.layer = layer;
+    p.layer_bytes = L.op_one;
     p.d = dsub;
     p.wbeta = wbeta();
     p.wphi = wphi();
@@ -1030,9 +1039,9 @@ struct Engine {
     // while that still leaves at least 4 blocks per SM
     const int blocks = (int)((L.HW + 127) / 128);
     int rpt = d.nray;
-    while (rpt > 1 && (long long)blocks * ((d.nray + rpt - 1) / rpt) < 608) rpt = (rpt + 1) / 2;
+    while (rpt > 1 && (long long)blocks * layers * ((d.nray + rpt - 1) / rpt) < 608) rpt = (rpt + 1) / 2;
     p.rays_per_thread = rpt;
-    dim3 grid((unsigned)blocks, (unsigned)((d.nray + rpt - 1) / rpt));
+    dim3 grid((unsigned)blocks, (unsigned)((d.nray + rpt - 1) / rpt), (unsigned)layers);
     mark_on(PROF_OP, s);
     p.wev02 = uniform_real() ? wev02() : nullptr;
     p.wevs = wevs();
@@ -1513,6 +1522,10 @@ struct Engine {
     if (st2 == nullptr) return DTMM_OK;
     int rc = wait_for(st2, st);  // inputs of the operators (setup, earlier passes)
     if (rc) return rc;
+    if (L.all_ops) {  // every layer in one launch
+      if ((rc = voxel_ops(0, ds[0], op_buffer(0, 0), st2, d.nlayers))) return rc;
+      return record(st2, f.ready[0]);
+    }
     const size_t n = L.cache_ops ? order.size() : std::min<size_t>(1, order.size());
     for (size_t q = 0; q < n; ++q)
       if ((rc = feed_one(q, order, ds, f))) return rc;
@@ -1533,6 +1546,10 @@ struct Engine {
     int rc;
     op = op_buffer(q, order[q]);
     if (L.cache_ops && pass > 0) return DTMM_OK;
+    if (L.all_ops && st2 != nullptr) {  // waited for once
+      if (q == 0) CK(cudaStreamWaitEvent(st, f.ready[0], 0));
+      return DTMM_OK;
+    }
     if (st2 == nullptr) return voxel_ops(order[q], ds[q], (cpx<R>*)op);
     if (!L.cache_ops && q + 1 < order.size() && (rc = feed_one(q + 1, order, ds, f))) return rc;
     CK(cudaStreamWaitEvent(st, f.ready[q], 0));

@@ -123,7 +123,8 @@ struct OpParams {
   long long ev_s[3];     // element strides of epsv over (layer, y, x) (0 = broadcast)
   long long ea_s[3];
   int eps_complex;
-  int layer;
+  int layer;             // first layer of the launch; blockIdx.z counts on from it
+  size_t layer_bytes;    // records of consecutive layers lie this far apart
   double d;              // sub-step thickness (pixels), direction not included
   const double* wbeta;   // [ray][nwin]
   const double* wphi;
@@ -290,8 +291,8 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
   const ff dd = ff_of(p.d);
   if (active) {
     const int y = pix / g.W, x = pix - y * g.W;
-    const long long eo = p.layer * p.ev_s[0] + y * p.ev_s[1] + x * p.ev_s[2];
-    const long long ao = p.layer * p.ea_s[0] + y * p.ea_s[1] + x * p.ea_s[2];
+    const long long eo = (p.layer + (int)blockIdx.z) * p.ev_s[0] + y * p.ev_s[1] + x * p.ev_s[2];
+    const long long ao = (p.layer + (int)blockIdx.z) * p.ea_s[0] + y * p.ea_s[1] + x * p.ea_s[2];
     const double* e = (const double*)p.epsv + eo;
     const double eo0 = e[0], ee = e[2], eps = p.uncorrected ? 0.0 : p.eps_dev[0];
     iso = eo0 == e[1] && e[1] == ee;
@@ -424,6 +425,7 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
 template <typename R, bool REAL, bool FOUR, bool BIAX>
 __global__ void k_voxel_op(OpParams p, Grid g, void* __restrict__ opv) {
   const int HW = g.H * g.W;
+  opv = (unsigned char*)opv + (size_t)blockIdx.z * p.layer_bytes;
   const int pix = blockIdx.x * blockDim.x + threadIdx.x;
   const int ray0 = blockIdx.y * p.rays_per_thread;
   const int ray1 = min(ray0 + p.rays_per_thread, p.nray);
@@ -433,8 +435,8 @@ __global__ void k_voxel_op(OpParams p, Grid g, void* __restrict__ opv) {
   }
   if (pix >= HW) return;
   const int y = pix / g.W, x = pix - y * g.W;
-  const long long eo = p.layer * p.ev_s[0] + y * p.ev_s[1] + x * p.ev_s[2];
-  const long long ao = p.layer * p.ea_s[0] + y * p.ea_s[1] + x * p.ea_s[2];
+  const long long eo = (p.layer + (int)blockIdx.z) * p.ev_s[0] + y * p.ev_s[1] + x * p.ev_s[2];
+  const long long ao = (p.layer + (int)blockIdx.z) * p.ea_s[0] + y * p.ea_s[1] + x * p.ea_s[2];
   const double theta = p.epsa[ao + 1], azim = p.epsa[ao + 2];
   if (p.eps_dev != nullptr) p.eps_eff = mk<double>(p.eps_dev[0], p.eps_dev[1]);
   constexpr int nrec = FOUR ? OP_REC : REC_BLOCK;
