@@ -550,6 +550,12 @@ struct Engine {
   // the block whose effective medium the k-space tables fetched now use
   int cur_blk = 0;
 
+  // Row and column passes as programmatic launches: in sweeps without an event
+  // between them (every operator ready), for grids of at most two waves, whose
+  // launch latency is a large part of their time.
+  bool pdl_sweep = false;
+  bool pdl_for(dim3 grid) const { return pdl_sweep && prof == nullptr && (size_t)grid.x * grid.y <= 1216; }
+
   // the line kernels take this side (fft_schedule 2 and 3 ask for the shared-memory passes)
   bool line_on(int n) const { return sizeof(R) == 8 && d.fft_schedule <= 1 && line_shape(n).maxl > 0; }
   bool row_line_on() const { return !row_reg() && line_on(d.width); }
@@ -620,6 +626,7 @@ struct Engine {
       p.tc = tx = std::min(tx, d.width);
       RegLaunch rl = col_reg_shape(d.height, cm * tx, st);
       rl.grid = dim3(band_tiles(p, tx), NI);
+      rl.pdl = pdl_for(rl.grid);
       mark(PROF_COL);
       // the diagonal table is cut at betamax: band variants of the transforms
       const int band = p.kop == KOP_DIAG && p.do_fwd && p.inverse_out ? col_band_pick(d.height, blimH_max) : 0;
@@ -651,6 +658,7 @@ struct Engine {
     rl.lim = std::max(0, std::min(blimH_max, d.height));
     const int nlaunch = band_tiles(p, tx);
     rl.grid = dim3(nlaunch, NI);
+    rl.pdl = pdl_for(rl.grid);
     mark(PROF_COL);
     const cudaError_t e = col_line(rl, p, g, in, out);
     mark(PROF_COL);
@@ -799,6 +807,7 @@ struct Engine {
       q.groups_inner = rec_bytes > ((size_t)64 << 20) ? 1 : 0;
       rl.grid = q.groups_inner ? dim3(d.nray * ngrp * npg, d.height) : dim3(d.height, d.nray * ngrp * npg);
       rl.st = st;
+      rl.pdl = pdl_for(rl.grid);
       mark(PROF_ROW);
       const int band = re ? row_band_pick(d.width, blim_max) : 0;
       const cudaError_t e = row_reg_dispatch(d.width, C, re, band, rl, q, g, Ub, Xb);
@@ -832,6 +841,7 @@ struct Engine {
     p.xr = 0;
     rl.lim = std::max(0, std::min(blim_max, d.width));
     rl.grid = p.groups_inner ? dim3(d.nray * ngrp * npg, d.height) : dim3(d.height, d.nray * ngrp * npg);
+    rl.pdl = pdl_for(rl.grid);
     mark(PROF_ROW);
     const cudaError_t e = row_line(C, re, rl, p, g, Ub, Xb);
     mark(PROF_ROW);
@@ -1539,6 +1549,9 @@ struct Engine {
     return record(st2, f.ready[q]);
   }
 
+  // no event between the passes from layer position q on
+  bool feed_quiet(int pass, size_t q) const { return q > 0 && L.cache_ops && (pass > 0 || (L.all_ops && st2 != nullptr)); }
+
   // before layer position q: its operators (computed now on the caller's
   // stream when there is no side stream), the next layer's queued beside it
   int feed_get(int pass, size_t q, const std::vector<int>& order, const std::vector<double>& ds, OpFeed& f,
@@ -1584,6 +1597,7 @@ struct Engine {
       const double ds = dsub[q];
       const void* op;
       if ((rc = feed_get(pass, q, order, dsub, feed, op))) return rc;
+      pdl_sweep = feed_quiet(pass, q);
       int kop;
       const void* ktab;
       const int bprev = cur_blk;
@@ -1628,6 +1642,7 @@ struct Engine {
     if ((rc = table(KT_D2, dir * dprev / 2, t2))) return rc;
     if ((rc = launch_col(cur, U, 4, 4, KOP_MAT, t2, 1, nullptr, true, true, 1.0 / d.height))) return rc;
     row_out = nullptr;
+    pdl_sweep = false;
     if ((rc = launch_rows(U, 4, true, 1.0 / d.width))) return rc;
     CK(cudaMemcpyAsync(F, U, sizeof(cpx<R>) * (size_t)NI * 4 * L.HW, cudaMemcpyDeviceToDevice, st));
     return DTMM_OK;
@@ -2033,6 +2048,7 @@ struct Engine {
         if (bulk && dir < 0 && (rc = bulk_add(l, -1, cur, -hd * dprev / 2, q > 0))) return rc;
         const void* op;
         if ((rc = feed_get(i, q, order, dsub, feed, op))) return rc;
+        pdl_sweep = feed_quiet(i, q);
         if (dir < 0) op = (const char*)op + back_records();
         int kop;
         const void* ktab;
@@ -2065,6 +2081,7 @@ struct Engine {
         dprev = ds;
         if (bulk && dir > 0 && (rc = bulk_add(l, 1, cur, hd * ds / 2, true))) return rc;
       }
+      pdl_sweep = false;
       if (dir > 0) {
         // exit: half step, interface effective -> n_out, windows and E -> H, into field_out
         const cpx<R>* t2;

@@ -27,6 +27,38 @@ namespace dtmm {
 constexpr int REC_BLOCK = 6;
 constexpr int OP_REC = 2 * REC_BLOCK;  // records of both blocks
 
+// Programmatic launches (RegLaunch::pdl, LineLaunch::pdl): the next kernel of
+// the stream may be scheduled while this one runs, and waits here until every
+// block of this one is done and its writes are visible.  Before the wait a
+// kernel reads only what was written before the sweep's first ordinary launch
+// (twiddles, wavenumbers, band limits).  Both are no-ops in ordinary launches.
+__device__ __forceinline__ void grid_wait() {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void grid_release() {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+
+// launch with a programmatic dependency on the stream's previous kernel
+template <typename K, typename... A>
+cudaError_t launch_with(bool pdl, K kern, dim3 grid, int threads, size_t smem, cudaStream_t st, A... a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, a...);
+}
+
 enum KOp { KOP_NONE = 0, KOP_DIAG = 1, KOP_MAT = 2 };
 
 struct Grid {

@@ -150,6 +150,8 @@ __global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
   // k0 of every wavelength, in turns per unit where the phases are formed in turns
   for (int gl = threadIdx.x; gl < G; gl += blockDim.x)
     s_kph[gl] = p.ks[lam0 + gl] * p.dir * (REAL ? 0.15915494309189533577 : 1.0);
+  grid_release();
+  grid_wait();  // the column pass's rows
   __syncthreads();
   const double sc = (double)p.in_scale;
   const int lineA = threadIdx.x / n1, tA = threadIdx.x - lineA * n1;
@@ -398,6 +400,8 @@ __global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
   const int lam = img_lam(g, img), ray = img_ray(g, img);
   const bool diag = p.kop == KOP_DIAG;
   bool band_x = true;  // the thread's column is read
+  grid_release();
+  grid_wait();  // the row pass's columns, and the readers of U
   if ((p.band_skip == 2 && diag) || p.xband) {  // tiles beyond the band: nothing is read from them, or zeros
     const int lim = (int)p.blim[lam];
     bool any = false;
@@ -581,6 +585,7 @@ struct LineLaunch {
   cudaStream_t st;
   LineGeom geom;
   int maxl, lim;  // lim: band limit of the transformed axis
+  bool pdl = false;  // programmatic dependency on the previous kernel (row and column passes)
 };
 
 #define DTMM_LINE_SIDES(X) \
@@ -603,8 +608,7 @@ template <typename K, typename... A>
 cudaError_t line_launch(K kern, const LineLaunch& L, A... a) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
   if (e != cudaSuccess) return e;
-  kern<<<L.grid, L.threads, L.smem, L.st>>>(a...);
-  return cudaGetLastError();
+  return launch_with(L.pdl, kern, L.grid, L.threads, L.smem, L.st, a...);
 }
 
 template <int C, bool REAL, int MAXL, int CN1, int CN2>

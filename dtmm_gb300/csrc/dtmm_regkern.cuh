@@ -141,6 +141,8 @@ __global__ void __launch_bounds__(XR > 0 ? (N1 * N2) / (XR > 0 ? XR : 1) : (N2 >
     s_lim[g2] = (int)p.blim[lam0 + g2];
   }
   const R sc = (R)p.in_scale;  // det of each block's records
+  grid_release();
+  grid_wait();  // the column pass's rows
   __syncthreads();
   const int line = threadIdx.x / N1, t = threadIdx.x % N1;
   const bool active = line < nlines;
@@ -449,6 +451,8 @@ __global__ void __launch_bounds__(col_max_threads(N), col_min_blocks(N))
   const int c = line / TX, kx = x0 + (line - c * TX);
   const bool in_x = kx < W;
   bool live = in_x;  // the column is read
+  grid_release();
+  grid_wait();  // the row pass's columns, and the readers of U
   if ((p.band_skip && p.kop == KOP_DIAG) || p.xband) {
     const int lim = (int)p.blim[lam];
     bool any = false;
@@ -615,6 +619,7 @@ struct RegLaunch {
   int threads;
   size_t smem;
   cudaStream_t st;
+  bool pdl = false;  // programmatic dependency on the previous kernel (row and column passes)
 };
 
 // row variants: every (C, REAL) for power-of-two sides, real records for the others
@@ -625,8 +630,7 @@ cudaError_t row_reg_variant(const RegLaunch& L, const RowParams& p, const Grid& 
   auto kern = k_layer_row_reg<float, C, REAL, N1, N2, BAND, XR>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
   if (e != cudaSuccess) return e;
-  kern<<<L.grid, L.threads, L.smem, L.st>>>(p, g, (const cpx<float>*)U, (cpx<float>*)X);
-  return cudaGetLastError();
+  return launch_with(L.pdl, kern, L.grid, L.threads, L.smem, L.st, p, g, (const cpx<float>*)U, (cpx<float>*)X);
 }
 
 // real records with a band variant b (row_band_pick), every (C, REAL) dense
@@ -673,8 +677,7 @@ cudaError_t col_reg_variant(const RegLaunch& L, const ColParams& p, const Grid& 
   auto kern = k_layer_col_reg<float, N, BAND>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
   if (e != cudaSuccess) return e;
-  kern<<<L.grid, L.threads, L.smem, L.st>>>(p, g, (const cpx<float>*)in, (cpx<float>*)out);
-  return cudaGetLastError();
+  return launch_with(L.pdl, kern, L.grid, L.threads, L.smem, L.st, p, g, (const cpx<float>*)in, (cpx<float>*)out);
 }
 
 // band variants (col_band_pick of the H axis) for the diagonal operator between
