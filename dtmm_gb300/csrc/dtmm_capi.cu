@@ -799,6 +799,8 @@ struct Engine {
       RegLaunch rl;
       rl.smem = smem;
       rl.threads = std::max(((nl * n1 + 31) / 32) * 32, 32);
+      // few short lines: a thread per pixel for the operators (up to 128)
+      if (q.xr <= 0) rl.threads = std::max(rl.threads, std::min(128, d.width / 32 * 32));
       const int ngrp = (d.nlam + p.G - 1) / p.G;
       const int npg = (d.npol + p.PB - 1) / p.PB;
       // one layer's operator records beyond half of L2 (128 MB): the groups of
