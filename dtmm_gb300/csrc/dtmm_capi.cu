@@ -26,6 +26,7 @@
 #include "../../include/dtmm_gb300.h"
 #include "dtmm_effmed.h"
 #include "dtmm_kernels.cuh"
+#include "dtmm_linef.cuh"
 #include "dtmm_linekern.cuh"
 #include "dtmm_regkern.cuh"
 
@@ -444,13 +445,35 @@ size_t part_bytes(int lines) {
   return (size_t)lines * kPartPitch * sizeof(unsigned);
 }
 
-// plain complex128 row transforms through the line kernels
+// launch shape and tile columns of the line kernels' column pass, NI images of
+// n-point columns, cm components, ny window rows; false: too large for a block
+template <typename R>
+bool col_line_shape(int n, int width, int NI, int cm, int ny, int col_tile, cudaStream_t st, LineLaunch& rl, int& tc) {
+  const LineShape ls = line_shape(n);
+  const int nmax = std::max(ls.n1, ls.n2);
+  const size_t per = (size_t)cm * n * sizeof(cpx<R>) * (ny > 1 ? 2 : 1);
+  const int most = sizeof(R) == 8 && ls.maxl <= 16 ? 128 : 256;  // the kernels' launch bounds
+  int tx = std::max(1, most / (cm * nmax));
+  while (tx > 1 && per * tx > 72 * 1024) tx /= 2;
+  // enough blocks for every SM
+  while (tx > 1 && (size_t)((width + tx - 1) / tx) * NI < 304) tx /= 2;
+  if (col_tile > 0 && col_tile * cm * nmax <= most && per * col_tile <= 180 * 1024) tx = col_tile;
+  tc = std::min(std::min(tx, width), kLineMax / cm);
+  rl = line_launch_of(ls, cm * tc, st);
+  rl.smem = per * tc + n * sizeof(cpx<R>) + (sizeof(R) == 8 ? part_bytes(cm * tc) : 0);
+  return rl.smem <= 220 * 1024;
+}
+
+// plain row transforms through the line kernels
+template <typename R>
 cudaError_t launch_rows_line(const LineShape& ls, const void* src, void* dst, int nlines, int W, bool inv,
                              const void* tw, double scale, cudaStream_t st) {
   const int lpb = std::min((ls.maxl <= 16 ? 128 : 256) / std::max(ls.n1, ls.n2), 16);
   LineLaunch L = line_launch_of(ls, lpb, st);
   L.grid = dim3((unsigned)((nlines + lpb - 1) / lpb));
-  L.smem = ((size_t)lpb * ls.n1 * L.geom.pitch + W) * sizeof(cpx<double>) + part_bytes(lpb);
+  L.smem = ((size_t)lpb * ls.n1 * L.geom.pitch + W) * sizeof(cpx<R>);
+  if (sizeof(R) == 4) return rows_linef(L, src, dst, nlines, W, inv, tw, scale, lpb);
+  L.smem += part_bytes(lpb);
   return rows_line(L, src, dst, nlines, W, inv, tw, scale, lpb);
 }
 
@@ -557,7 +580,7 @@ struct Engine {
   bool pdl_for(dim3 grid) const { return pdl_sweep && prof == nullptr && (size_t)grid.x * grid.y <= 1216; }
 
   // the line kernels take this side (fft_schedule 2 and 3 ask for the shared-memory passes)
-  bool line_on(int n) const { return sizeof(R) == 8 && d.fft_schedule <= 1 && line_shape(n).maxl > 0; }
+  bool line_on(int n) const { return d.fft_schedule <= 1 && line_shape(n).maxl > 0; }
   bool row_line_on() const { return !row_reg() && line_on(d.width); }
 
   // the buffer that holds a row pass's band-limited output, if any
@@ -581,7 +604,7 @@ struct Engine {
       }
     }
     if (line_on(d.width)) {
-      const cudaError_t e = launch_rows_line(line_shape(d.width), data, data, nlines, d.width, inv, P(L.twW), scale, st);
+      const cudaError_t e = launch_rows_line<R>(line_shape(d.width), data, data, nlines, d.width, inv, P(L.twW), scale, st);
       ++launches;
       if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_rows_line: %s", cudaGetErrorString(e));
       return DTMM_OK;
@@ -640,27 +663,15 @@ struct Engine {
 
   // column pass through the line kernels
   int launch_col_line(ColParams& p, const cpx<R>* in, cpx<R>* out) {
-    const LineShape ls = line_shape(d.height);
-    const int cm = std::max(p.cin, p.cout), nmax = std::max(ls.n1, ls.n2);
-    const size_t per = (size_t)cm * d.height * sizeof(cpx<R>) * (p.ny > 1 ? 2 : 1);
-    const int most = ls.maxl <= 16 ? 128 : 256;  // the kernel's launch bounds
-    int tx = std::max(1, most / (cm * nmax));
-    while (tx > 1 && per * tx > 72 * 1024) tx /= 2;
-    // enough blocks for every SM
-    while (tx > 1 && (size_t)((d.width + tx - 1) / tx) * NI < 304) tx /= 2;
-    if (d.col_tile > 0 && d.col_tile * cm * nmax <= most && per * d.col_tile <= 180 * 1024) tx = d.col_tile;
-    tx = std::min(std::min(tx, d.width), kLineMax / cm);
-    if (per * tx + d.height * sizeof(cpx<R>) > 220 * 1024)
+    LineLaunch rl;
+    if (!col_line_shape<R>(d.height, d.width, NI, std::max(p.cin, p.cout), p.ny, d.col_tile, st, rl, p.tc))
       return fail(DTMM_ENOTSUP, "column of %d pixels too large for one block", d.height);
-    p.tc = tx;
-    LineLaunch rl = line_launch_of(ls, cm * tx, st);
-    rl.smem = per * tx + d.height * sizeof(cpx<R>) + part_bytes(cm * tx);
     rl.lim = std::max(0, std::min(blimH_max, d.height));
-    const int nlaunch = band_tiles(p, tx);
+    const int nlaunch = band_tiles(p, p.tc);
     rl.grid = dim3(nlaunch, NI);
     rl.pdl = pdl_for(rl.grid);
     mark(PROF_COL);
-    const cudaError_t e = col_line(rl, p, g, in, out);
+    const cudaError_t e = sizeof(R) == 8 ? col_line(rl, p, g, in, out) : col_linef(rl, p, g, in, out);
     mark(PROF_COL);
     ++launches;
     if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_col_line: %s", cudaGetErrorString(e));
@@ -791,7 +802,7 @@ struct Engine {
       // in registers; one window: in place
       q.xr = re && xr_pixels(d.width) > 0 && nl == kXrLines && p.PB <= 2 && d.nlam % p.G == 0 && d.npol % p.PB == 0
                  ? 1 : 0;
-      if (re && (L.nwin == 1 || p.win_only >= 0)) q.xr = -1;
+      if (re && L.nwin == 1) q.xr = -1;
       const size_t smem = (q.xr != 0 ? 1 : 2) * (size_t)nl * reg_row_stride(n1, d.width) * sizeof(cpx<R>) +
                           d.width * sizeof(cpx<R>);
       if (smem > 220 * 1024 || nl * n1 > reg_row_max_threads(d.width))
@@ -824,7 +835,10 @@ struct Engine {
   int launch_row_line(RowParams& p, const cpx<R>* Ub, cpx<R>* Xb, int C, bool re) {
     const LineShape ls = line_shape(d.width);
     const int nmax = std::max(ls.n1, ls.n2), most = ls.maxl <= 16 ? 128 : 256;
-    const size_t line_bytes = 2 * (size_t)ls.n1 * line_row_pitch(ls, re) * sizeof(cpx<R>);
+    // one window of complex64 rows: the operators in place, no second set of lines
+    p.xr = sizeof(R) == 4 && L.nwin == 1 ? -1 : 0;
+    const int pitch = sizeof(R) == 8 ? line_row_pitch(ls, re) : (ls.n2 | 1);
+    const size_t line_bytes = (p.xr < 0 ? 1 : 2) * (size_t)ls.n1 * pitch * sizeof(cpx<R>);
     p.PB = d.npol;
     if (p.PB * C * nmax > most || p.PB * C * line_bytes > 200 * 1024 || p.PB * C > kLineMax) p.PB = 1;
     const int perG = p.PB * C;
@@ -834,18 +848,17 @@ struct Engine {
     p.G = std::min(G, d.nlam);
     const int nl = p.G * perG;
     LineLaunch rl = line_launch_of(ls, nl, st);
-    rl.smem = nl * line_bytes + d.width * sizeof(cpx<R>) + part_bytes(nl);
+    rl.smem = nl * line_bytes + d.width * sizeof(cpx<R>) + (sizeof(R) == 8 ? part_bytes(nl) : 0);
     if (rl.smem > 220 * 1024) return fail(DTMM_ENOTSUP, "row of %d pixels too large for one block", d.width);
     const int ngrp = (d.nlam + p.G - 1) / p.G, npg = (d.npol + p.PB - 1) / p.PB;
     // one layer's operator records beyond half of L2: the groups of a row next to each other
     const size_t rec_bytes = (re ? sizeof(R) : sizeof(cpx<R>)) * (size_t)d.nray * L.nwin * p.rec_stride * L.HW;
     p.groups_inner = rec_bytes > ((size_t)64 << 20) ? 1 : 0;
-    p.xr = 0;
     rl.lim = std::max(0, std::min(blim_max, d.width));
     rl.grid = p.groups_inner ? dim3(d.nray * ngrp * npg, d.height) : dim3(d.height, d.nray * ngrp * npg);
     rl.pdl = pdl_for(rl.grid);
     mark(PROF_ROW);
-    const cudaError_t e = row_line(C, re, rl, p, g, Ub, Xb);
+    const cudaError_t e = sizeof(R) == 8 ? row_line(C, re, rl, p, g, Ub, Xb) : row_linef(C, re, rl, p, g, Ub, Xb);
     mark(PROF_ROW);
     ++launches;
     if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_row_line: %s", cudaGetErrorString(e));
@@ -2499,10 +2512,15 @@ int diffract_impl(int H, int W, int nimg, int nlam, const void* dmat, const void
   int lpb = std::max(1, std::min(16, 4096 / W));
   size_t smem = (size_t)lpb * W * sizeof(cpx<R>) + W * (sizeof(cpx<R>) + sizeof(int));
   if (smem > 220 * 1024) return fail(DTMM_ENOTSUP, "row of %d pixels too large for one block", W);
+  const LineShape lsW = line_shape(W), lsH = line_shape(H);
   if (rrows) {
     const cudaError_t e = fft_rows_reg_dispatch(W, false, rl, in, X, nlines, twW, 1.0f);
     ++launches;
     if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_fft_rows_reg: %s", cudaGetErrorString(e));
+  } else if (lsW.maxl > 0) {
+    const cudaError_t e = launch_rows_line<R>(lsW, in, X, nlines, W, false, twW, 1.0, st);
+    ++launches;
+    if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_rows_line: %s", cudaGetErrorString(e));
   } else {
     CK(cudaFuncSetAttribute(k_fft_rows<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_fft_rows<R, false><<<(nlines + lpb - 1) / lpb, 256, smem, st>>>((const cpx<R>*)in, X, nlines, W, pW, twW,
@@ -2541,6 +2559,12 @@ int diffract_impl(int H, int W, int nimg, int nlam, const void* dmat, const void
     const cudaError_t e = col_reg_dispatch(H, 0, cl, p, g, X, out);
     ++launches;
     if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_layer_col_reg: %s", cudaGetErrorString(e));
+  } else if (LineLaunch ll; lsH.maxl > 0 && col_line_shape<R>(H, W, nimg, 4, 1, 0, st, ll, p.tc)) {
+    ll.lim = H;
+    ll.grid = dim3((W + p.tc - 1) / p.tc, nimg);
+    const cudaError_t e = sizeof(R) == 8 ? col_line(ll, p, g, X, out) : col_linef(ll, p, g, X, out);
+    ++launches;
+    if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_col_line: %s", cudaGetErrorString(e));
   } else {
     const size_t per = 4 * (size_t)H * sizeof(cpx<R>) * 2;
     int tc = 1;
@@ -2558,6 +2582,10 @@ int diffract_impl(int H, int W, int nimg, int nlam, const void* dmat, const void
     const cudaError_t e = fft_rows_reg_dispatch(W, true, rl, out, out, nlines, twW, (float)(1.0 / W));
     ++launches;
     if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_fft_rows_reg: %s", cudaGetErrorString(e));
+  } else if (lsW.maxl > 0) {
+    const cudaError_t e = launch_rows_line<R>(lsW, out, out, nlines, W, true, twW, 1.0 / W, st);
+    ++launches;
+    if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_rows_line: %s", cudaGetErrorString(e));
   } else {
     smem = (size_t)lpb * W * sizeof(cpx<R>) + W * (sizeof(cpx<R>) + sizeof(int));
     CK(cudaFuncSetAttribute(k_fft_rows<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

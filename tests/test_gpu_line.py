@@ -93,6 +93,35 @@ def test_register_columns_match_shared_memory_passes(height, method, diffraction
     assert np.linalg.norm(a - b) <= 3e-6 * np.linalg.norm(b)
 
 
+@pytest.mark.parametrize("shape", [(7, 2), (24, 30), (45, 50), (100, 210), (250, 330), (200, 125), (500, 300), (150, 64),
+                                   (64, 150), (12, 900)])
+@pytest.mark.parametrize("method,diffraction,pixelsize", [("4x4", 3, 50.0), ("2x2", 1, 100.0), ("4x4", 1, 220.0)])
+def test_run_time_lengths_match_shared_memory_passes(shape, method, diffraction, pixelsize):
+    """complex64 passes of run-time lengths, alone and beside register passes (one side each), with the
+    same bound as the register columns."""
+    a = _mixed(shape, method, diffraction, 0, pixelsize)
+    b = _mixed(shape, method, diffraction, 2, pixelsize)
+    assert np.linalg.norm(a - b) <= 3e-6 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("shape", [(45, 50), (96, 100), (150, 64), (64, 64), (250, 330)])
+@pytest.mark.parametrize("precision,tol", [("double", 2e-14), ("mixed", 3e-6)])
+def test_refocus_matches_fft(shape, precision, tol):
+    """diffract with a random matrix per k against torch.fft in complex128 (two transforms and a 4x4
+    product: the bounds above)."""
+    import torch
+
+    from dtmm_gb300 import pom
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    f = torch.randn((2, 3, 4) + shape + (2,), generator=g, device="cuda", dtype=torch.float64)
+    f = torch.view_as_complex(f)
+    m = torch.view_as_complex(torch.randn((3,) + shape + (4, 4, 2), generator=g, device="cuda", dtype=torch.float64))
+    ref = torch.fft.ifft2(torch.einsum("lhwij,pljhw->plihw", m, torch.fft.fft2(f)))
+    out = pom.diffract(f if precision == "double" else f.to(torch.complex64), m)
+    assert float((out - ref).norm() / ref.norm()) <= tol
+
+
 @pytest.mark.parametrize("shape", [(64, 50), (150, 96)])
 def test_line_passes_read_no_column_beyond_the_band(shape):
     import torch
