@@ -452,7 +452,7 @@ bool col_line_shape(int n, int width, int NI, int cm, int ny, int col_tile, cuda
   const LineShape ls = line_shape(n);
   const int nmax = std::max(ls.n1, ls.n2);
   const size_t per = (size_t)cm * n * sizeof(cpx<R>) * (ny > 1 ? 2 : 1);
-  const int most = sizeof(R) == 8 && ls.maxl <= 16 ? 128 : 256;  // the kernels' launch bounds
+  const int most = sizeof(R) == 8 ? line_most(ls, true) : 256;  // the kernels' launch bounds
   int tx = std::max(1, most / (cm * nmax));
   while (tx > 1 && per * tx > 72 * 1024) tx /= 2;
   // enough blocks for every SM
@@ -834,13 +834,14 @@ struct Engine {
   // row pass through the line kernels: about 8 lines a block
   int launch_row_line(RowParams& p, const cpx<R>* Ub, cpx<R>* Xb, int C, bool re) {
     const LineShape ls = line_shape(d.width);
-    const int nmax = std::max(ls.n1, ls.n2), most = ls.maxl <= 16 ? 128 : 256;
+    const int nmax = std::max(ls.n1, ls.n2), most = line_most(ls, sizeof(R) == 8 && re);
+    const size_t room = most == 160 ? 104 * 1024 : 200 * 1024;  // two blocks of the former on a SM
     // one window of complex64 rows: the operators in place, no second set of lines
     p.xr = sizeof(R) == 4 && L.nwin == 1 ? -1 : 0;
     const int pitch = sizeof(R) == 8 ? line_row_pitch(ls, re) : (ls.n2 | 1);
     const size_t line_bytes = (p.xr < 0 ? 1 : 2) * (size_t)ls.n1 * pitch * sizeof(cpx<R>);
     p.PB = d.npol;
-    if (p.PB * C * nmax > most || p.PB * C * line_bytes > 200 * 1024 || p.PB * C > kLineMax) p.PB = 1;
+    if (p.PB * C * nmax > most || p.PB * C * line_bytes > room || p.PB * C > kLineMax) p.PB = 1;
     const int perG = p.PB * C;
     int G = std::max(1, std::min(8 / perG, most / (perG * nmax)));
     if (d.row_group > 0) G = d.row_group;

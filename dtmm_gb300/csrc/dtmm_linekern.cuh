@@ -42,6 +42,24 @@ constexpr int kLineMax = 64;  // lines of a block at most
 
 // slot of (k, m): a compile-time power-of-two n2 swizzles (no padding, three
 // 256-point blocks of eight complex128 lines a SM instead of two), others pad
+// Launch bounds: the largest block and the blocks of a SM, by the points a thread
+// holds (maxl) and the side (cn1 maxl; cn1 0: run-time lengths).  The passes wait
+// on shared memory and on 64-bit multiplies, so warps in flight count for more than
+// spills to L1: 12 warps of 168 registers a SM as 3 x 128 threads, or 10 as 2 x 160
+// where that holds eight lines of 18 or 20 points a thread.  Against one block of
+// 256 threads at 255 registers (5 to 8 warps), ten layers, row pass: side 300, one
+// window 2.16 -> 1.35 ms, nine windows 14.0 -> 9.5; side 125 3.64 -> 2.81 and 24.5 ->
+// 17.6; side 432 4.14 -> 3.61 and 28.6 -> 23.7 (its column pass 2.22 -> 2.63).  Four
+// blocks at 128 registers for up to 12 points lost up to 9 % (side 120, 144).
+// Above 520 points shared memory leaves one or two such blocks, and the run-time
+// kernels spill four times as much at 168 registers (1024 points: 199 -> 209 ms).
+constexpr int line_threads(int maxl, int cn1) {
+  return maxl <= 16 ? 128 : (cn1 == 0 || cn1 * maxl > 520 ? 256 : (maxl <= 20 ? 160 : 128));
+}
+constexpr int line_blocks(int maxl, int cn1) {
+  return line_threads(maxl, cn1) == 128 ? 3 : (line_threads(maxl, cn1) == 160 ? 2 : 1);
+}
+
 template <int CN2>
 __host__ __device__ __forceinline__ constexpr int line_pitch(int n2) {
   return CN2 != 0 && is_pow2(CN2) ? n2 : (n2 | 1);
@@ -120,7 +138,7 @@ __device__ __forceinline__ cpx<T> swapc(cpx<T> a) {
 // ray.  Threads: lines x max(n1, n2).
 // ---------------------------------------------------------------------------
 template <int C, bool REAL, int MAXL, int CN1, int CN2>
-__global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
+__global__ void __launch_bounds__(line_threads(MAXL, CN1), line_blocks(MAXL, CN1))
     k_row_line(RowParams p, Grid g, LineGeom s, int limW, const cpx<double>* __restrict__ U,
                cpx<double>* __restrict__ X) {
   using T = typename std::conditional<REAL, double, cpx<double>>::type;
@@ -311,7 +329,7 @@ __global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
 // lines a block.
 // ---------------------------------------------------------------------------
 template <int MAXL>
-__global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
+__global__ void __launch_bounds__(line_threads(MAXL, 0), line_blocks(MAXL, 0))
     k_rows_line(const cpx<double>* src, cpx<double>* dst, int nlines, int W, LineGeom s, int inv,
                 const cpx<double>* __restrict__ twg, double scale, int lpb) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -385,7 +403,7 @@ __global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
 // with |frequency index| along y beyond it are zero after a KOP_DIAG table.
 // ---------------------------------------------------------------------------
 template <int MAXL, int CN1, int CN2>
-__global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
+__global__ void __launch_bounds__(line_threads(MAXL, CN1), line_blocks(MAXL, CN1))
     k_col_line(ColParams p, Grid g, LineGeom s, int limH, const cpx<double>* __restrict__ X,
                cpx<double>* __restrict__ U) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -571,12 +589,14 @@ __global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 3 : 1)
 }
 
 // ---------------------------------------------------------------------------
-// Launch glue.  Sides whose two factors lie in {8, 10, 12, 15, 16} have row (real
-// operator records) and column kernels with n1 x n2 known at compile time,
-// instantiated in dtmm_line_<a..d>.cu: no switch, hardly a spill (256-point rows,
-// nine windows, 0.90 ms a layer against 1.08 ms; 128-point rows, one window, 58
-// us against 69; 64-point columns 17 us against 27).  Every other
-// side takes the run-time kernels of dtmm_line_any*.cu.
+// Launch glue.  The sides of DTMM_LINE_SIDES (the most even splits n1 n2 of the
+// sides grids are usually chosen at, 45 to 1024) have row (real operator records) and
+// column kernels with n1 x n2 known at compile time, instantiated in
+// dtmm_line_<a..o>.cu: no switch and few spills, so that more blocks fit a SM.
+// Ten layers, run-time lengths -> these (row / column pass, ms): side 48, one window
+// .28 / .33 -> .21 / .24; 112, nine windows 6.9 / 1.24 -> 5.3 / .99; 200 14.4 / 3.2 ->
+// 6.6 / 1.6; 320 19.0 / 4.2 -> 11.3 / 2.1; 512 38.2 / 8.5 -> 32.3 / 6.5; 1024 199 / 29.7 ->
+// 170 / 24.0.  Every other side takes the run-time kernels of dtmm_line_any*.cu.
 // ---------------------------------------------------------------------------
 struct LineLaunch {
   dim3 grid;
@@ -589,8 +609,11 @@ struct LineLaunch {
 };
 
 #define DTMM_LINE_SIDES(X) \
-  X(8, 8) X(8, 10) X(8, 12) X(8, 16) X(10, 10) X(10, 12) X(10, 15) X(10, 16) X(12, 12) X(12, 15) X(12, 16) X(15, 15) \
-  X(15, 16) X(16, 16)
+  X(5, 9) X(5, 10) X(5, 15) X(5, 25) X(6, 8) X(6, 10) X(7, 9) X(7, 25) X(8, 8) X(8, 9) X(8, 10) X(8, 12) \
+  X(8, 14) X(8, 16) X(9, 10) X(9, 15) X(10, 10) X(10, 11) X(10, 12) X(10, 14) X(10, 15) X(10, 16) X(10, 20) \
+  X(10, 25) X(11, 20) X(12, 12) X(12, 14) X(12, 15) X(12, 16) X(14, 14) X(14, 15) X(14, 16) X(14, 20) X(14, 25) \
+  X(15, 15) X(15, 16) X(15, 18) X(15, 20) X(15, 22) X(16, 16) X(16, 18) X(16, 20) X(16, 21) X(16, 22) X(16, 24) \
+  X(16, 28) X(16, 32) X(18, 20) X(18, 24) X(20, 20) X(20, 24) X(20, 32) X(32, 32)
 
 inline bool line_side(int n1, int n2) {
 #define DTMM_LINE_IS(A, B) \
@@ -598,6 +621,10 @@ inline bool line_side(int n1, int n2) {
   DTMM_LINE_SIDES(DTMM_LINE_IS)
 #undef DTMM_LINE_IS
   return false;
+}
+// threads a row (complex records: real = false) or column kernel's block may have
+inline int line_most(const LineShape& ls, bool real) {
+  return real && line_side(ls.n1, ls.n2) ? line_threads(ls.n2, ls.n1) : line_threads(ls.maxl, 0);
 }
 // slots of a row kernel's line per n1: what line_pitch gives there
 inline int line_row_pitch(const LineShape& ls, bool real) {

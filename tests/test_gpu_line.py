@@ -140,3 +140,15 @@ def test_line_passes_read_no_column_beyond_the_band(shape):
     plan.workspace.fill_(255)
     plan.run(fin, again)
     assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("shape", [(48, 50), (60, 72), (75, 90), (112, 135), (140, 168), (196, 210), (224, 200),
+                                   (270, 288), (300, 320), (400, 384), (48, 512), (512, 48), (45, 63), (110, 125),
+                                   (175, 220), (250, 280), (330, 336), (350, 352), (360, 432), (448, 480), (32, 640),
+                                   (640, 32), (1024, 32)])
+@pytest.mark.parametrize("method,diffraction", [("4x4", 3), ("2x2", 1)])
+def test_line_passes_of_compile_time_sides(shape, method, diffraction):
+    # the further sides with kernels of their own, rows and columns, the tolerance above
+    a = _run(shape, method, diffraction, 0)
+    b = _run(shape, method, diffraction, 2)
+    assert np.linalg.norm(a - b) <= 2e-14 * np.linalg.norm(b)
