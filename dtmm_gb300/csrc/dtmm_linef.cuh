@@ -1,12 +1,18 @@
 // Row and column passes of a layer step, complex64 bulk, for the sides without
 // a register transform of their own (dtmm_regkern.cuh): any n = n1 n2 with n1,
-// n2 up to 32 (`line_shape`), two steps of register DFTs of run-time length.
-// Slots, threads and steps are those of dtmm_linekern.cuh, in FP32 arithmetic.
+// n2 up to 32 (`line_shape`), two steps of register DFTs.  Slots, threads and
+// steps are those of dtmm_linekern.cuh, in FP32 arithmetic.  The sides of
+// DTMM_LINEF_SIDES have n1 and n2 at compile time: no switch over lengths, index
+// arithmetic by constants and no spills at fewer registers.
 //
 // In shared-memory mixed-radix passes (prime by prime, every column of the
 // grid, the whole band) 330-point rows of 8 images took 114 us a layer and
-// 250-point columns 72 us; here 66 and 43 us (a launch is two to three waves of
-// blocks of 128 registers: latency).
+// 250-point columns 72 us; with run-time lengths 66 and 44 us; at compile time 33
+// and 30 us (a launch is two to three waves of blocks: latency, and in the first
+// step of 10 x 25 three of five threads wait).  Twenty layers, seven rays, run-time
+// lengths -> compile time (row / column pass, ms): side 48 .46 / .39 -> .36 / .28; 100
+// 1.60 / .79 -> .93 / .60; 200 8.6 / 4.0 -> 4.3 / 2.3; 300 6.6 / 3.4 -> 3.5 / 2.3; 350 6.5 /
+// 3.0 -> 3.3 / 2.1.
 #pragma once
 
 #include <type_traits>
@@ -15,6 +21,20 @@
 
 namespace dtmm {
 
+// Launch bounds.  Threads follow the length class that `line_shape` chose the side by;
+// blocks a SM as many as the registers allow with few spills.  Rows of 22 and 25 points
+// a thread spill at 80 registers and still gain by three blocks of 256 threads instead
+// of two (side 350, seven rays 4.24 -> 3.31 ms, three window rows 3.30 -> 2.80), their
+// columns lose (2.10 -> 2.43).  Eight blocks of 128 threads instead of six for up to 12
+// points: 5 % faster for one window, 3 % slower for nine.
+constexpr int linef_threads(int maxl, int cn1, int cn2) {
+  return maxl <= 16 && (cn1 == 0 || (line_len_ok(cn1, 16) && line_len_ok(cn2, 16))) ? 128 : 256;
+}
+constexpr int linef_row_blocks(int maxl, int cn1, int cn2) {
+  return linef_threads(maxl, cn1, cn2) == 128 ? (cn1 ? 6 : 5) : (cn1 ? 3 : 2);
+}
+constexpr int linef_col_blocks(int maxl, int cn1) { return maxl <= (cn1 ? 20 : 16) ? 3 : 2; }
+
 // W^(t k) at k n1 + t
 __device__ __forceinline__ void linef_tw(cpx<float>* tw, const void* twg, int n, int n1) {
   for (int e = threadIdx.x; e < n; e += blockDim.x) tw[e] = ((const cpx<float>*)twg)[(e % n1) * (e / n1)];
@@ -22,13 +42,14 @@ __device__ __forceinline__ void linef_tw(cpx<float>* tw, const void* twg, int n,
 
 // Row pass (see RowParams): one row of G wavelengths x PB polarisations of one
 // ray.  Threads: lines x max(n1, n2).  p.xr < 0: one window, in place.
-template <int C, bool REAL, int MAXL>
-__global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 5 : 2)
+template <int C, bool REAL, int MAXL, int CN1, int CN2>
+__global__ void __launch_bounds__(linef_threads(MAXL, CN1, CN2), linef_row_blocks(MAXL, CN1, CN2))
     k_row_linef(RowParams p, Grid g, LineGeom s, int limW, const cpx<float>* __restrict__ U, cpx<float>* __restrict__ X) {
   using T = typename std::conditional<REAL, float, cpx<float>>::type;
   __shared__ float s_kph[kLineMax];
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n1 = s.n1, n2 = s.n2, H = g.H, W = g.W, P = s.pitch, LS = n1 * P;
+  const int n1 = CN1 ? CN1 : s.n1, n2 = CN1 ? CN2 : s.n2, H = g.H, W = CN1 ? CN1 * CN2 : g.W;
+  const int P = CN1 ? (CN2 | 1) : s.pitch, LS = n1 * P;
   const int ngrp = (g.nlam + p.G - 1) / p.G, npg = (g.npol + p.PB - 1) / p.PB;
   const int y = p.groups_inner ? blockIdx.y : blockIdx.x;
   const int gi = p.groups_inner ? blockIdx.x : blockIdx.y;
@@ -107,7 +128,7 @@ __global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 5 : 2)
             v[m] = rl[o + st * m];
           }
         }
-        line_dft<float, MAXL>(v, len);
+        step_dft<MAXL, CN1, CN2>(v, roleA, len);
         if (half == 0) {
           const int wo = fwd ? t * n1 : t, ws = fwd ? 1 : n1;
           const int o = fwd ? t : P * t, st = fwd ? P : 1;
@@ -233,11 +254,11 @@ __global__ void __launch_bounds__(MAXL <= 16 ? 128 : 256, MAXL <= 16 ? 5 : 2)
 // Column pass (see ColParams): tc columns x max(cin, cout) components of one
 // image; tile element (slot, line) at slot * lines + line, slot m + n2 t for
 // ky = t + n1 m.  limH: entries beyond it along y are zero after a KOP_DIAG table.
-template <int MAXL>
-__global__ void __launch_bounds__(256, MAXL <= 16 ? 3 : 2)
+template <int MAXL, int CN1, int CN2>
+__global__ void __launch_bounds__(256, linef_col_blocks(MAXL, CN1))
     k_col_linef(ColParams p, Grid g, LineGeom s, int limH, const cpx<float>* __restrict__ X, cpx<float>* __restrict__ U) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n1 = s.n1, n2 = s.n2, H = g.H, W = g.W, TX = p.tc;
+  const int n1 = CN1 ? CN1 : s.n1, n2 = CN1 ? CN2 : s.n2, H = CN1 ? CN1 * CN2 : g.H, W = g.W, TX = p.tc;
   const int CM = max(p.cin, p.cout), NL = CM * TX;
   const int img = blockIdx.y;
   const int tile = (p.tile_lo > 0 && (int)blockIdx.x >= p.tile_lo) ? p.tile_hi0 + ((int)blockIdx.x - p.tile_lo)
@@ -319,7 +340,7 @@ __global__ void __launch_bounds__(256, MAXL <= 16 ? 3 : 2)
           v[m] = z[st * m];
         }
       }
-      if (!skip_dft) line_dft<float, MAXL>(v, len);
+      if (!skip_dft) step_dft<MAXL, CN1, CN2>(v, roleA, len);
       if (half == 0 && !skip_dft) {
         const int wo = fwd ? t * n1 : t, ws = fwd ? 1 : n1;
         cpx<float>* z = tile_x + (size_t)(fwd ? t : n2 * t) * NL + line;
@@ -389,6 +410,24 @@ __global__ void __launch_bounds__(256, MAXL <= 16 ? 3 : 2)
     if (!(fwd && half == 1 && p.kop != KOP_MAT)) __syncthreads();
   }
 }
+
+// Sides with kernels of their own (real operator records), instantiated in dtmm_linef_<a..d>.cu
+#define DTMM_LINEF_SIDES(X) \
+  X(5, 9) X(5, 10) X(5, 15) X(5, 25) X(6, 8) X(6, 10) X(7, 9) X(7, 25) X(8, 9) X(9, 10) X(9, 15) X(10, 10) \
+  X(10, 11) X(10, 12) X(10, 14) X(10, 15) X(10, 20) X(10, 25) X(11, 20) X(12, 14) X(12, 15) X(14, 14) X(14, 15) \
+  X(14, 20) X(14, 25) X(15, 15) X(15, 18) X(15, 20) X(15, 22) X(16, 22) X(18, 20)
+#define DTMM_LINEF_DECLARE(A, B)                                                                                     \
+  cudaError_t row_linef_##A##_##B(int C, const LineLaunch& L, const RowParams& p, const Grid& g, const void* U, void* X); \
+  cudaError_t col_linef_##A##_##B(const LineLaunch& L, const ColParams& p, const Grid& g, const void* in, void* out);
+#define DTMM_LINEF_DEFINE(A, B)                                                                                      \
+  cudaError_t row_linef_##A##_##B(int C, const LineLaunch& L, const RowParams& p, const Grid& g, const void* U, void* X) { \
+    return line_launch(C == 4 ? k_row_linef<4, true, B, A, B> : k_row_linef<2, true, B, A, B>, L, p, g, L.geom, L.lim, \
+                       (const cpx<float>*)U, (cpx<float>*)X);                                                        \
+  }                                                                                                                  \
+  cudaError_t col_linef_##A##_##B(const LineLaunch& L, const ColParams& p, const Grid& g, const void* in, void* out) { \
+    return line_launch(k_col_linef<B, A, B>, L, p, g, L.geom, L.lim, (const cpx<float>*)in, (cpx<float>*)out);       \
+  }
+DTMM_LINEF_SIDES(DTMM_LINEF_DECLARE)
 
 cudaError_t row_linef(int C, bool real, const LineLaunch& L, const RowParams& p, const Grid& g, const void* U, void* X);
 cudaError_t col_linef(const LineLaunch& L, const ColParams& p, const Grid& g, const void* in, void* out);

@@ -5,9 +5,13 @@
 namespace dtmm {
 
 cudaError_t col_linef(const LineLaunch& L, const ColParams& p, const Grid& g, const void* in, void* out) {
+#define DTMM_LINEF_COL(A, B) \
+  if (L.geom.n1 == A && L.geom.n2 == B) return col_linef_##A##_##B(L, p, g, in, out);
+  DTMM_LINEF_SIDES(DTMM_LINEF_COL)
+#undef DTMM_LINEF_COL
   if (L.maxl <= 16)
-    return line_launch(k_col_linef<16>, L, p, g, L.geom, L.lim, (const cpx<float>*)in, (cpx<float>*)out);
-  return line_launch(k_col_linef<32>, L, p, g, L.geom, L.lim, (const cpx<float>*)in, (cpx<float>*)out);
+    return line_launch(k_col_linef<16, 0, 0>, L, p, g, L.geom, L.lim, (const cpx<float>*)in, (cpx<float>*)out);
+  return line_launch(k_col_linef<32, 0, 0>, L, p, g, L.geom, L.lim, (const cpx<float>*)in, (cpx<float>*)out);
 }
 
 cudaError_t rows_linef(const LineLaunch& L, const void* src, void* dst, int nlines, int W, bool inv, const void* tw,

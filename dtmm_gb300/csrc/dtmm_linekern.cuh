@@ -40,8 +40,6 @@ struct LineGeom {
 
 constexpr int kLineMax = 64;  // lines of a block at most
 
-// slot of (k, m): a compile-time power-of-two n2 swizzles (no padding, three
-// 256-point blocks of eight complex128 lines a SM instead of two), others pad
 // Launch bounds: the largest block and the blocks of a SM, by the points a thread
 // holds (maxl) and the side (cn1 maxl; cn1 0: run-time lengths).  The passes wait
 // on shared memory and on 64-bit multiplies, so warps in flight count for more than
@@ -60,6 +58,8 @@ constexpr int line_blocks(int maxl, int cn1) {
   return line_threads(maxl, cn1) == 128 ? 3 : (line_threads(maxl, cn1) == 160 ? 2 : 1);
 }
 
+// slot of (k, m): a compile-time power-of-two n2 swizzles (no padding, three
+// 256-point blocks of eight complex128 lines a SM instead of two), others pad
 template <int CN2>
 __host__ __device__ __forceinline__ constexpr int line_pitch(int n2) {
   return CN2 != 0 && is_pow2(CN2) ? n2 : (n2 | 1);
@@ -73,17 +73,17 @@ __device__ __forceinline__ int line_slot(int k, int m, int pitch) {
 }
 
 // the DFT of a step: n1 x n2 known at compile time (CN1 > 0) or run-time lengths
-template <int MAXL, int CN1, int CN2>
-__device__ __forceinline__ void step_dft(cpx<fx> (&v)[MAXL], bool roleA, int len) {
+template <int MAXL, int CN1, int CN2, typename R = fx>
+__device__ __forceinline__ void step_dft(cpx<R> (&v)[MAXL], bool roleA, int len) {
   if constexpr (CN1 == 0) {
-    line_dft<fx, MAXL>(v, len);
+    line_dft<R, MAXL>(v, len);
   } else if constexpr (CN1 == CN2) {
-    RegDFTg<fx, CN1, false>::run(v);
+    RegDFTg<R, CN1, false>::run(v);
   } else {
     if (roleA)
-      RegDFTg<fx, CN2, false>::run(v);
+      RegDFTg<R, CN2, false>::run(v);
     else
-      RegDFTg<fx, CN1, false>::run(v);
+      RegDFTg<R, CN1, false>::run(v);
   }
 }
 

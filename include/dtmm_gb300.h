@@ -37,8 +37,8 @@ extern "C" {
    (dtmm/propagate_4x4.py:515-560); 4x4, any reflection mode, any npass */
 #define DTMM_DIFFRACTION_FULL (-1)
 
-#define DTMM_PRECISION_MIXED 0  /* complex64 bulk, FP64 eigen-solve and operator tables */
-#define DTMM_PRECISION_DOUBLE 1 /* complex128 bulk (the reference's default precision)  */
+#define DTMM_PRECISION_MIXED 0  /* complex64 bulk, FP64 k-space tables, eigen-solve in FP64 or FP32 pairs (48 bits) */
+#define DTMM_PRECISION_DOUBLE 1 /* complex128 bulk (the reference's default precision), lines transformed in 64-bit block fixed point */
 
 typedef struct dtmm_transfer_desc {
   /* grid and images: images = nray * npol * nlam, in the reference's
@@ -73,17 +73,18 @@ typedef struct dtmm_transfer_desc {
   const double* beta;      /* [nray]                                            */
   const double* phi;       /* [nray]                                            */
   /* upper bound on the bytes of cached per-layer operators (npass > 1 reuses
-     them across passes when they fit); 0 selects the default (48 GiB) */
+     them across passes when they fit; one-pass stacks of one block whose
+     records take at most 32 MB form every layer's in one launch); 0 selects
+     the default (48 GiB) */
   size_t op_cache_bytes;
   /* 1: the caller guarantees real eps whose every eigenvalue (and hence the
      effective medium) exceeds max(betamax, beta)^2; every radicand of the
-     eigen-solve is then positive and the engine uses real FP64 arithmetic and
+     eigen-solve is then positive and the engine uses real arithmetic and
      half-size operator records.  Ignored for complex eps. */
   int real_path;
   /* tuning (0 = built-in choice; results do not depend on row_group and
      col_tile): wavelengths per row block, columns per column block, and the
-     line transform schedule: 1 = two-step register transform where it
-     applies (power-of-two sides 64..1024, complex64), 2 = shared-memory
+     line transform schedule: 1 = two-step transforms in registers, 2 = shared-memory
      mixed radix with radix-4 passes first, 3 = the same with radix-8 first */
   int row_group;
   int col_tile;
@@ -231,7 +232,7 @@ int dtmm_transfer_timed(const dtmm_transfer_desc* desc, const dtmm_transfer_io* 
      before any stream capture.
    - Transfers whose workspace (dtmm_transfer_workspace_size) exceeds the
      array are rejected with DTMM_ENOSPACE and a message giving both sizes;
-     an npass > 1 transfer whose every-layer operator cache does not fit is
+     a transfer whose every-layer operator cache does not fit is
      first retried with two alternating operator buffers (same results).
    - The first call on a stream creates that stream's side stream, as
      dtmm_transfer does; later calls on it create nothing.

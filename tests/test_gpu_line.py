@@ -152,3 +152,17 @@ def test_line_passes_of_compile_time_sides(shape, method, diffraction):
     a = _run(shape, method, diffraction, 0)
     b = _run(shape, method, diffraction, 2)
     assert np.linalg.norm(a - b) <= 2e-14 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("shape", [(45, 48), (60, 50), (63, 72), (90, 75), (100, 110), (125, 120), (135, 140), (168, 150),
+                                   (175, 180), (200, 196), (210, 220), (250, 225), (270, 280), (330, 300), (350, 352),
+                                   (45, 360), (360, 45)])
+@pytest.mark.parametrize("swap", [False, True])
+@pytest.mark.parametrize("method,diffraction,pixelsize", [("4x4", 3, 50.0), ("2x2", 1, 220.0)])
+def test_compile_time_lines_match_shared_memory_passes(shape, swap, method, diffraction, pixelsize):
+    """complex64 passes of the sides with line kernels of their own, each as rows and as columns, with the
+    same bound as the register columns."""
+    shape = shape[::-1] if swap else shape
+    a = _mixed(shape, method, diffraction, 0, pixelsize)
+    b = _mixed(shape, method, diffraction, 2, pixelsize)
+    assert np.linalg.norm(a - b) <= 3e-6 * np.linalg.norm(b)
