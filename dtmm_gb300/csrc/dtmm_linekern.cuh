@@ -125,8 +125,8 @@ __device__ __forceinline__ cpx<double> line_out(cpx<fx> a, int emax, int guard) 
 }
 
 // exp(i arg k): k in turns for real FP64 arguments
-__device__ __forceinline__ cpx<double> line_phase(double arg, double k) { return turn_of(arg * k); }
-__device__ __forceinline__ cpx<double> line_phase(cpx<double> arg, double k) { return phase_of<double>(arg, k); }
+__device__ __forceinline__ cpx<double> line_phase(double arg, double k, int rest) { return turn_of(arg * k, rest); }
+__device__ __forceinline__ cpx<double> line_phase(cpx<double> arg, double k, int) { return phase_of<double>(arg, k); }
 
 template <typename T>
 __device__ __forceinline__ cpx<T> swapc(cpx<T> a) {
@@ -143,6 +143,7 @@ __global__ void __launch_bounds__(line_threads(MAXL, CN1), line_blocks(MAXL, CN1
                cpx<double>* __restrict__ X) {
   using T = typename std::conditional<REAL, double, cpx<double>>::type;
   __shared__ double s_kph[kLineMax];
+  __shared__ int s_krest[kLineMax];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_scale[kLineMax];  // emax << 8 | second-step guard bits of each line
   const int n1 = CN1 ? CN1 : s.n1, n2 = CN2 ? CN2 : s.n2;
@@ -166,8 +167,12 @@ __global__ void __launch_bounds__(line_threads(MAXL, CN1), line_blocks(MAXL, CN1
   for (int e = threadIdx.x; e < W; e += blockDim.x) tw[e] = line_tw(((const cpx<double>*)p.tw)[(e % n1) * (e / n1)]);
   for (int e = threadIdx.x; e < nlines * LS; e += blockDim.x) acc[e] = mk<double>(0, 0);
   // k0 of every wavelength, in turns per unit where the phases are formed in turns
-  for (int gl = threadIdx.x; gl < G; gl += blockDim.x)
-    s_kph[gl] = p.ks[lam0 + gl] * p.dir * (REAL ? 0.15915494309189533577 : 1.0);
+  for (int gl = threadIdx.x; gl < G; gl += blockDim.x) {
+    const double k = p.ks[lam0 + gl] * p.dir;
+    const TurnScale t = REAL ? turn_scale(k) : TurnScale{k, 0};
+    s_kph[gl] = t.k;
+    s_krest[gl] = t.rest;
+  }
   grid_release();
   grid_wait();  // the column pass's rows
   __syncthreads();
@@ -291,14 +296,15 @@ __global__ void __launch_bounds__(line_threads(MAXL, CN1), line_blocks(MAXL, CN1
       const T* eb = rec + (C == 4 ? REC_BLOCK : 0);
       for (int gl = 0; gl < G; ++gl) {
         const double kph = s_kph[gl];
+        const int kr = s_krest[gl];
         cpx<double> qf, dpf, qb, dpb;
         {
-          const cpx<double> f0 = line_phase(ef[4], kph), f1 = line_phase(ef[5], kph);
+          const cpx<double> f0 = line_phase(ef[4], kph, kr), f1 = line_phase(ef[5], kph, kr);
           qf = f1 * sc;
           dpf = f0 - f1;
         }
         if (C == 4) {
-          const cpx<double> b0 = line_phase(eb[4], kph), b1 = line_phase(eb[5], kph);
+          const cpx<double> b0 = line_phase(eb[4], kph, kr), b1 = line_phase(eb[5], kph, kr);
           qb = b1 * sc;
           dpb = b0 - b1;
         }

@@ -168,8 +168,28 @@ static void check_turns() {
   if (!(worst <= 1.2e-16L) || !nan) g_bad = 1;
 }
 
+// exp(i k a) through turns: the rounding of u = a k / (2 pi) alone, 2^-53 of it (and
+// 2^-61, the part of the scale's rest that is cut off), beside the turn's own error
+static void check_scaled_turns() {
+  const long double pi = acosl(-1.0L);
+  unsigned s = 7;
+  long double worst = 0;
+  for (int i = 0; i < 400000; ++i) {
+    const double scale[4] = {0.05, 1.0, 30.0, 1e3};
+    const double k = (i & 4 ? -1.0 : 1.0) * (0.1 + std::fabs(rnd(s)) * 5.0), a = rnd(s) * scale[i & 3];
+    const TurnScale t = turn_scale(k);
+    const cpx<double> e = turn_of(a * t.k, t.rest);
+    const long double x = (long double)a * k, u = fabsl(x / (2 * pi));
+    const long double bound = 1.2e-16L + 2 * pi * u * 1.01L / 9007199254740992.0L;
+    worst = std::fmax(worst, std::fmax(fabsl(e.re - cosl(x)), fabsl(e.im - sinl(x))) / bound);
+  }
+  std::printf("scaled_turn_err %.3Lf of the bound\n", worst);
+  if (!(worst <= 1.0L)) g_bad = 1;
+}
+
 int main() {
   check_turns();
+  check_scaled_turns();
   for (int n = 2; n <= 1024; ++n) {
     if (line_shape(n).maxl == 0) continue;
     if (n > 400 && n % 16 && n != 405 && n != 450 && n != 500 && n != 750) continue;
