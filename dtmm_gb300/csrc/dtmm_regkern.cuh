@@ -79,8 +79,10 @@ __host__ __device__ constexpr int row_band_pick(int n, int lim) {
 // W / XR threads, and each thread keeps the accumulators of its XR pixels in
 // registers across the windows: no second set of lines and no shared-memory
 // read-modify-write per window (nine windows, one layer: 128 points 40 -> 31 us,
-// 256 points of the 2x2 method 66 -> 48 us).
-// XR = -1: one window (no windows, or a single-window chain).  There is nothing
+// 256 points of the 2x2 method 66 -> 48 us).  Four 128-thread blocks a SM: five at 96
+// registers spill next to nothing and are slower (256 points of the 4x4 method 95 ->
+// 101 us a launch, 128 points 29 -> 34), six at 80 as well (99, 38): shared memory bounds it.
+// XR = -1: one window (one window in all).  There is nothing
 // to accumulate: the operators' results replace the transformed rows in place,
 // without the second set of lines (half the shared memory, so twice the blocks
 // a SM) and its clearing, reads and writes.  320 points, 70
