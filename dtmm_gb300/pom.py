@@ -11,7 +11,7 @@ does the three steps in one pass per pixel.
 
 Arrays may be numpy (copied to the device and back) or CUDA tensors (results
 stay on the device).  ``pmat`` and ``cmf`` may be device tensors; host ones are
-copied in stream order without waiting for queued work.  The small jones / 4x4
+staged and copied in stream order without waiting for queued work.  The small jones / 4x4
 matrices are built on the host (``jonesvec``, ``polarizer``,
 ``rotated_matrix``, ``ray_jonesmat4x4``).
 Refocusing goes through a per-k diffraction matrix (``diffract``, the
@@ -153,10 +153,22 @@ def _dev_field(field):
     return torch.from_numpy(np.ascontiguousarray(a, dtype)).cuda(), True
 
 
-def _upload(a, device):
-    """A small host array on the device, in stream order: the copy is staged before the call returns, and
-    the work queued before it is not waited for."""
-    return _torch().from_numpy(np.ascontiguousarray(a)).to(device, non_blocking=True)
+def _upload(arrays, device):
+    """Small host arrays of doubles on the device, ordered on the current stream without waiting for the work
+    queued there: one copy from page-locked memory of torch's caching host allocator, which keeps it until the
+    copy is done, so the caller's arrays are free when this returns.  Refused in a capture, whose replays would
+    copy from host memory that is gone by then."""
+    torch = _torch()
+    if torch.cuda.is_current_stream_capturing():
+        raise RuntimeError("host arrays cannot be uploaded while a graph is captured: pass device tensors")
+    flat = [a.reshape(-1).view(np.float64) for a in arrays]
+    at = np.cumsum([0] + [-(-len(a) // 32) * 32 for a in flat])  # each on a 256-byte boundary
+    staged = torch.empty(int(at[-1]), dtype=torch.float64, pin_memory=True)
+    host = staged.numpy()
+    for o, a in zip(at, flat):
+        host[o:o + len(a)] = a
+    dev = staged.to(device, non_blocking=True)
+    return [dev[o:o + len(a)] for o, a in zip(at.tolist(), flat)]
 
 
 def _dev_real(x, device):
@@ -181,14 +193,22 @@ def _stream(device):
     return ctypes.c_void_p(_torch().cuda.current_stream(device).cuda_stream)
 
 
-def _desc(f, jvec, pmat, window):
-    """Descriptor for a field tensor [..., (2,) lam, 4, H, W]; returns (desc, keep-alive list, leading shape)."""
+def _small(a, dtype, tdtype, device):
+    """A tensor of the given dtype on the device, or a host array that has to be uploaded."""
+    torch = _torch()
+    if isinstance(a, torch.Tensor):  # already on the device: no upload behind queued work
+        return a.to(device=device, dtype=tdtype).contiguous()
+    return np.ascontiguousarray(a, dtype)
+
+
+def _desc(f, jvec, pmat, window, cmf=None):
+    """Descriptor for a field tensor [..., (2,) lam, 4, H, W]; returns (desc, keep-alive list, leading shape); with
+    ``cmf`` the colour matching table leads the list."""
     torch = _torch()
     h, w = f.shape[-2:]
     nlam = f.shape[-4]
     d = _lib.PomDesc()
     d.height, d.width, d.nlam = int(h), int(w), int(nlam)
-    keep = []
     if jvec is not None:
         if f.ndim < 5 or f.shape[-5] != 2:
             raise ValueError("Invalid field shape.")
@@ -200,15 +220,22 @@ def _desc(f, jvec, pmat, window):
         lead = tuple(f.shape[:-4])
         d.npol = 1
     d.nset = int(np.prod(lead)) if lead else 1
+    small = []
+    if cmf is not None:
+        c = _small(cmf, np.float64, torch.float64, f.device)
+        if tuple(c.shape) != (int(nlam), 3):
+            raise ValueError("cmf must have one row per wavelength")
+        small.append(c)
     if pmat is not None:
-        if isinstance(pmat, torch.Tensor):  # already on the device: no upload behind queued work
-            pt = pmat.to(device=f.device, dtype=torch.complex128).contiguous()
-        else:
-            pt = _upload(np.asarray(pmat, np.complex128), f.device)
-        if tuple(pt.shape) != (4, 4):
+        p = _small(pmat, np.complex128, torch.complex128, f.device)
+        if tuple(p.shape) != (4, 4):
             raise NotImplementedError("one 4x4 analyzer matrix for every pixel and wavelength")
-        keep.append(pt)
-        d.pmat = pt.data_ptr()
+        small.append(p)
+    host = [a for a in small if isinstance(a, np.ndarray)]
+    sent = iter(_upload(host, f.device) if host else ())
+    keep = [next(sent) if isinstance(a, np.ndarray) else a for a in small]
+    if pmat is not None:
+        d.pmat = keep[-1].data_ptr()
     if window is not None:
         wt = _dev_real(window, f.device)
         if tuple(wt.shape) != (h, w):
@@ -388,24 +415,31 @@ def specter2color(spec, cmf, norm=False, gamma=True, gray=False, out=None):
 def pom_image(field, cmf, jvec=None, pmat=None, window=None, norm=False, gamma=True, gray=False, stream=None):
     """The POM image of a transferred field in one pass: polarizer (``jvec``
     over the x / y axis), window, analyzer ``pmat``, Poynting summed over
-    every leading set, XYZ, colour -> float32 [H, W, 3]."""
+    every leading set, XYZ, colour -> float32 [H, W, 3].
+
+    ``stream`` (a raw handle; default the current stream) takes the uploads and
+    the kernel; device inputs must be ready there, and the image is."""
     torch = _torch()
+    if stream is not None:
+        device = field.device if isinstance(field, torch.Tensor) and field.is_cuda else torch.device(
+            "cuda", torch.cuda.current_device())
+        caller = torch.cuda.current_stream(device)
+        if int(stream) != caller.cuda_stream:
+            with torch.cuda.stream(torch.cuda.ExternalStream(int(stream), device=device)):
+                rgb = pom_image(field, cmf, jvec, pmat, window, norm, gamma, gray)
+            if isinstance(rgb, torch.Tensor):
+                rgb.record_stream(caller)  # read there as well
+            return rgb
     f, host = _dev_field(field)
-    d, keep, lead = _desc(f, jvec, pmat, window)
-    if isinstance(cmf, torch.Tensor):  # already on the device: no upload behind queued work
-        c = cmf.to(device=f.device, dtype=torch.float64).contiguous()
-    else:
-        c = _upload(np.asarray(cmf, np.float64), f.device)
-    if tuple(c.shape) != (f.shape[-4], 3):
-        raise ValueError("cmf must have one row per wavelength")
+    d, keep, lead = _desc(f, jvec, pmat, window, cmf)
+    c = keep[0]
     rgb = torch.empty(tuple(f.shape[-2:]) + (3,), dtype=torch.float32, device=f.device)
     mode, val = _norm_args(norm)
     lib = _lib.load()
-    st = ctypes.c_void_p(stream) if stream is not None else _stream(f.device)
     _lib.check(lib.dtmm_pom_image(ctypes.byref(d), ctypes.c_void_p(f.data_ptr()), ctypes.c_void_p(c.data_ptr()),
                                   mode, val, _gamma_arg(gamma), int(bool(gray)), ctypes.c_void_p(rgb.data_ptr()),
-                                  st))
-    rgb._dtmm_keep = (keep, c)
+                                  _stream(f.device)))
+    rgb._dtmm_keep = keep
     return rgb.cpu().numpy() if host else rgb
 
 
