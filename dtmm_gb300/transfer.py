@@ -323,7 +323,8 @@ def _joined(blocks, shape):
 class _Material:
     """Optical data resident on the device (uploaded once per call, or kept by
     the caller): one block, or several joined along the layers with the block
-    of every layer (each block keeps its own effective medium)."""
+    of every layer (each block keeps its own effective medium).  The director
+    angles' copy may be in flight when the constructor returns: ``wait``."""
 
     def __init__(self, blocks, shape, device, block_sym=None, block_eff=None):
         import torch
@@ -345,9 +346,13 @@ class _Material:
         # (read-only views of broadcast data are copied: torch wants writeable memory)
         ev = _writeable(np.ascontiguousarray(ev, np.complex128 if self.eps_complex else np.float64))
         self.epsv = torch.from_numpy(ev).to(device)
-        self.epsa = torch.from_numpy(_writeable(np.ascontiguousarray(ea, np.float64))).to(device, non_blocking=True)
-        # biaxial voxels take the general eigen-solve (complex FP64 path); many voxels are looked
-        # through on the device (128 x 128 x 60 voxels: 2.3 ms less a call), few on the host
+        ea = _writeable(np.ascontiguousarray(ea, np.float64))
+        self.epsa = torch.from_numpy(ea).to(device, non_blocking=True)
+        landed = torch.cuda.Event()
+        landed.record(torch.cuda.current_stream(device))
+        self._landing = (landed, ea)
+        # biaxial voxels take the general eigen-solve (complex FP64 path); beside the angles' copy many
+        # voxels are looked through on the device (128 x 128 x 60 voxels: 2.3 ms less a call), few on the host
         # (48 x 48 x 12: 0.08 ms less than there)
         if ev.size < 1 << 18:
             flat = ev.reshape(-1, 3)
@@ -359,6 +364,12 @@ class _Material:
             self.eps_min = float(flat.min()) if not self.eps_complex else None
         self.thickness = np.asarray(d, np.float64)
         self.nlayers = L
+
+    def wait(self):
+        """Wait for the last upload: from then on any stream may read the material, and the host arrays are free."""
+        if self._landing is not None:
+            self._landing[0].synchronize()
+            self._landing = None
 
 
 class DeviceMaterial:
@@ -624,6 +635,7 @@ def plan_transfer(field_shape, wavelengths, pixelsize, optical_data, beta=0.0, p
     else:
         od, bs, be = effective_blocks(validate_optical_data(optical_data, shape), eff_data)
         mat = _Material(od, shape, dev, bs, be)
+        mat.wait()
     beta = np.asarray(beta, np.float64)
     nray = 1 if beta.ndim == 0 else len(beta)
     nlam = field_shape[-4]
@@ -747,30 +759,33 @@ def _transfer_single(field_in, wavelengths, pixelsize, optical_data, beta, phi, 
     nimg = int(np.prod(field_in.shape[:-3]))
     npol = nimg // (nray * nlam)
     mat = _Material(od, shape, dev, block_sym, block_eff)
-    fdev = field_dev.to(cdt).contiguous()
-    L = mat.nlayers
-    bulk_dev = None
-    if ret_bulk:
-        bulk_dev = torch.zeros((L + 2,) + tuple(field_in.shape), dtype=cdt, device=dev)
-        bulk_dev[0] = fdev
-        fin_dev = bulk_dev[0]
-        fout_dev = bulk_dev[-1]
-        out_given = 0
-        if out is not None and method == "4x4":  # 2x2 zeroes the caller's out (dtmm/transfer.py:1054)
-            ob = np.asarray(out)
-            bulk_dev[-1] = torch.from_numpy(np.ascontiguousarray(ob[-1], np.complex128)).to(dev).to(cdt)
-            out_given = 1
-    else:
-        fin_dev = fdev
-        if out is not None and method == "4x4":
-            fout_dev = torch.from_numpy(np.ascontiguousarray(out, np.complex128)).to(dev).to(cdt).contiguous()
-            out_given = 1
-        else:
-            fout_dev = torch.empty_like(fdev)
+    try:
+        fdev = field_dev.to(cdt).contiguous()
+        L = mat.nlayers
+        bulk_dev = None
+        if ret_bulk:
+            bulk_dev = torch.zeros((L + 2,) + tuple(field_in.shape), dtype=cdt, device=dev)
+            bulk_dev[0] = fdev
+            fin_dev = bulk_dev[0]
+            fout_dev = bulk_dev[-1]
             out_given = 0
-    plan = DevicePlan(field_in.shape, mat, ks, beta, phi, nray, npol, nlam, method, diffraction, reflection, npass,
-                      nstep, betamax, nin, nout, smooth, precision, dev, norm=norm)
-    plan.run(fin_dev, fout_dev, bulk=bulk_dev, out_given=out_given)
+            if out is not None and method == "4x4":  # 2x2 zeroes the caller's out (dtmm/transfer.py:1054)
+                ob = np.asarray(out)
+                bulk_dev[-1] = torch.from_numpy(np.ascontiguousarray(ob[-1], np.complex128)).to(dev).to(cdt)
+                out_given = 1
+        else:
+            fin_dev = fdev
+            if out is not None and method == "4x4":
+                fout_dev = torch.from_numpy(np.ascontiguousarray(out, np.complex128)).to(dev).to(cdt).contiguous()
+                out_given = 1
+            else:
+                fout_dev = torch.empty_like(fdev)
+                out_given = 0
+        plan = DevicePlan(field_in.shape, mat, ks, beta, phi, nray, npol, nlam, method, diffraction, reflection, npass,
+                          nstep, betamax, nin, nout, smooth, precision, dev, norm=norm)
+        plan.run(fin_dev, fout_dev, bulk=bulk_dev, out_given=out_given)
+    finally:
+        mat.wait()  # (the transfer is queued behind the upload)
     if ret_bulk:
         res = _new_host(bulk_dev)
         if out is not None:

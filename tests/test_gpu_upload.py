@@ -84,3 +84,39 @@ def test_pom_image_host_arrays_are_refused_in_a_capture():
     with torch.cuda.graph(g, stream=s):
         with pytest.raises(RuntimeError, match="device tensors"):
             pom.pom_image(f, cmf, jvec=(0.6, 0.8), pmat=pmat)
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("voxel_eps", [False, True])
+def test_plan_owns_its_material_when_the_call_returns(pinned, voxel_eps):
+    """A plan from host arrays, made on a busy stream and run on another one: the director angles are on the
+    device and the caller's arrays free.  One eps for the sample is looked through on the host, 2^18 values
+    (88 x 100 x 10 voxels) and more on the device."""
+    import torch
+
+    from dtmm_gb300 import samples
+    from dtmm_gb300.illumination import illumination_device
+    from dtmm_gb300.transfer import plan_transfer
+
+    shape, wl = (100, 88), [500.0]
+    d, ev, ea = samples.twisted_nematic(shape, 10, no=1.52, ne=1.71, amplitude=0.3, seed=3)
+    ea = np.array(np.broadcast_to(ea, (10,) + shape + (3,)))
+    if voxel_eps:
+        ev = np.array(np.broadcast_to(ev, (10,) + shape + (3,)))
+    fin = illumination_device(shape, wl, 100.0, precision="mixed")
+    opts = dict(method="4x4", diffraction=1, npass=1, precision="mixed")
+    want = torch.empty_like(fin)
+    plan_transfer(tuple(fin.shape), wl, 100.0, [(d, ev, ea.copy())], **opts).run(fin, want)
+    torch.cuda.synchronize()
+    t = torch.from_numpy(ea)
+    mine = (t.pin_memory() if pinned else t.clone()).numpy()
+    got = torch.empty_like(fin)
+    _spoil(ea.size)
+    other = torch.cuda.Stream()
+    torch.cuda._sleep(BUSY)
+    plan = plan_transfer(tuple(fin.shape), wl, 100.0, [(d, ev, mine)], **opts)
+    mine[...] = np.nan
+    with torch.cuda.stream(other):
+        plan.run(fin, got)
+    other.synchronize()
+    assert torch.equal(got, want)
