@@ -506,8 +506,9 @@ class DevicePlan:
 
         ``row_group``/``col_tile`` change only how work is split into blocks
         (results are bit-identical); ``fft_schedule`` 1/2/3 selects the
-        register two-step transform, radix-4-first or radix-8-first shared
-        memory passes (results agree to rounding).
+        two-step transforms in registers (sides that do not split take shared
+        memory), radix-4-first or radix-8-first shared memory passes (results
+        agree to rounding).
         """
         self.desc.fft_schedule = int(fft_schedule)
         self.desc.row_group = int(row_group)

@@ -2,8 +2,9 @@
 
 The engine exposes three knobs per transfer (``DevicePlan.set_tuning``):
 
-* ``fft_schedule`` -- how each row/column line is transformed: 1 = the
-  two-step register transform (power-of-two sides 64..1024, complex64),
+* ``fft_schedule`` -- how each row/column line is transformed: 1 = two-step
+  transforms in registers, in either precision and for every side that splits
+  into two factors the library transforms (others take shared memory),
   2 = shared-memory mixed-radix passes with radix 4 first, 3 = the same with
   radix 8 first (fewer passes through shared memory for sides divisible by 8);
 * ``row_group`` -- wavelengths per row block (lines resident per block);
@@ -16,7 +17,8 @@ so results are bit-identical across them; the schedules agree to rounding.
 same grid and image axes (a few layers of the plan's own material) and keeps
 the fastest, by coordinate descent: schedule first, then row group, then
 column tile.  Results are cached per key (grid, method, precision, windows,
-fields per wavelength) in memory and, optionally, in a JSON file.
+fields per wavelength, kind of operator records, generation of the passes) in
+memory and, optionally, in a JSON file.
 """
 from __future__ import annotations
 
@@ -25,26 +27,35 @@ import os
 
 import numpy as np
 
-# sides with a register line transform (the library's reg_lanes table); for
-# sides that are not powers of two it covers real operator records only
+# sides with complex64 kernels of their own (the library's reg_lanes table); for
+# sides that are not powers of two they cover real operator records only.  Every
+# other side that splits takes the line kernels, as complex128 sides do.
 SIDES_REG = (64, 80, 96, 112, 128, 144, 160, 192, 224, 240, 256, 288, 320, 336, 384, 400, 432, 448, 480, 512, 1024)
+
+
+# Generation of the passes that the knobs choose among: picks stored for earlier
+# ones (before the line kernels, schedule 1 was none of their candidates) lapse.
+PASSES = 2
 
 
 def tuning_key(plan):
     d = plan.desc
-    return "%dx%d/m%d/%s/d%d/f%d" % (d.height, d.width, d.method, plan.precision,
-                                     max(1, d.diffraction), d.npol * d.nray)
+    return "%dx%d/m%d/%s%s/d%d/f%d/p%d" % (d.height, d.width, d.method, plan.precision, "" if d.real_path else "/complex",
+                                           max(1, d.diffraction), d.npol * d.nray, PASSES)
 
 
 def schedules(plan):
+    """Line-transform schedules to time: the two-step transforms, then the shared-memory passes."""
     d = plan.desc
-    out = []
-    if plan.precision != "double" and (d.height in SIDES_REG or d.width in SIDES_REG):
-        out.append(1)
-    out.append(2)
-    if d.height % 8 == 0 or d.width % 8 == 0:
-        out.append(3)
-    return out
+    return [1, 2] + ([3] if d.height % 8 == 0 or d.width % 8 == 0 else [])
+
+
+def col_tiles(plan, schedule):
+    """Column tiles to time (0 = the engine's choice): a two-step column block holds at most 16 lines, four
+    columns of the 4x4 method's components or eight of the 2x2 method's, so wider tiles are the same launch."""
+    if schedule != 1:
+        return [0, 1, 2, 4, 8, 16]
+    return [0, 1, 2, 4] + ([8] if plan.desc.method == 2 else [])
 
 
 class Autotuner:
@@ -123,7 +134,7 @@ class Autotuner:
         best["fft_schedule"] = min(cands, key=lambda s: measure(dict(best, fft_schedule=s)))
         groups = [0] + [gg for gg in (1, 2, 3, 4, 6, 8) if gg <= d.nlam]
         best["row_group"] = min(groups, key=lambda gg: measure(dict(best, row_group=gg)))
-        tiles = [0, 1, 2, 4, 8] + ([16] if best["fft_schedule"] != 1 else [])
+        tiles = col_tiles(target, best["fft_schedule"])
         best["col_tile"] = min(tiles, key=lambda t: measure(dict(best, col_tile=t)))
         torch.cuda.synchronize(target.device)
         self.cache[key] = dict(best)
@@ -155,4 +166,4 @@ def proxy_plan_device(plan, mat, spec, precision, device, layers=2, **options):
                          phi=spec["phi"], precision=precision, device=device, **options)
 
 
-__all__ = ["Autotuner", "tuning_key", "proxy_plan", "proxy_plan_device", "schedules"]
+__all__ = ["Autotuner", "tuning_key", "proxy_plan", "proxy_plan_device", "schedules", "col_tiles"]
