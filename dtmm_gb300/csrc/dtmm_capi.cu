@@ -1072,11 +1072,16 @@ struct Engine {
     p.wev02 = uniform_real() ? wev02() : nullptr;
     p.wevs = wevs();
     p.wc2 = wc2();
-    if (real_ops()) {
+    if (real_ops() && sizeof(R) == 4) {
       if (p.four)
-        k_voxel_op<R, true, true, false><<<grid, 128, 0, s>>>(p, g, op);
+        k_voxel_op_lean<true><<<grid, 128, 0, s>>>(p, g, op);
       else
-        k_voxel_op<R, true, false, false><<<grid, 128, 0, s>>>(p, g, op);
+        k_voxel_op_lean<false><<<grid, 128, 0, s>>>(p, g, op);
+    } else if (real_ops()) {
+      if (p.four)
+        k_voxel_op<double, true, true, false><<<grid, 128, 0, s>>>(p, g, op);
+      else
+        k_voxel_op<double, true, false, false><<<grid, 128, 0, s>>>(p, g, op);
     } else if (d.biaxial) {
       if (p.four)
         k_voxel_op<R, false, true, true><<<grid, 128, 0, s>>>(p, g, op);

@@ -278,17 +278,8 @@ __host__ __device__ __forceinline__ TurnScale turn_scale(double k) {
   return t;
 }
 
-// (cos, sin) of u (1 + rest 2^-83) turns in Q62; u finite
-__host__ __device__ __forceinline__ cpx<fx> fx_turn(double u, int rest = 0) {
-  const long long b = dbits(u);
-  const int sh = ((int)(b >> 52) & 0x7ff) - 1011;  // 2^64 u = significand << sh
-  const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffULL) | (1ULL << 52);
-  unsigned long long f;
-  if (sh >= 0)
-    f = sh < 64 ? (m << sh) + (unsigned long long)(madw((int)(m >> 22), rest, 0) >> (sh < 61 ? 61 - sh : 0)) : 0;
-  else
-    f = sh > -55 ? ((m >> (-sh - 1)) + 1) >> 1 : 0;
-  if (b < 0) f = 0 - f;
+// (cos, sin) of f / 2^64 turns in Q62
+__host__ __device__ __forceinline__ cpx<fx> fx_turn_at(unsigned long long f) {
   const unsigned i = (unsigned)((f + (1ULL << (63 - kTurnBits))) >> (64 - kTurnBits)) & ((1u << kTurnBits) - 1u);
   const long long r = (long long)(f - ((unsigned long long)i << (64 - kTurnBits)));
   constexpr long long kPi4 = 3622009729038561421LL;  // pi / 4 in Q62
@@ -308,6 +299,42 @@ __host__ __device__ __forceinline__ cpx<fx> fx_turn(double u, int rest = 0) {
 #endif
   const cpx<fx> e = mk<fx>(fx(-cm, 0), fx(sn, 0)) * cs;  // 2^68
   return mk<fx>(fx(cs.re.v + ((e.re.v + 32) >> 6), 0), fx(cs.im.v + ((e.im.v + 32) >> 6), 0));
+}
+
+// (cos, sin) of u (1 + rest 2^-83) turns in Q62; u finite
+__host__ __device__ __forceinline__ cpx<fx> fx_turn(double u, int rest = 0) {
+  const long long b = dbits(u);
+  const int sh = ((int)(b >> 52) & 0x7ff) - 1011;  // 2^64 u = significand << sh
+  const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffULL) | (1ULL << 52);
+  unsigned long long f;
+  if (sh >= 0)
+    f = sh < 64 ? (m << sh) + (unsigned long long)(madw((int)(m >> 22), rest, 0) >> (sh < 61 ? 61 - sh : 0)) : 0;
+  else
+    f = sh > -55 ? ((m >> (-sh - 1)) + 1) >> 1 : 0;
+  if (b < 0) f = 0 - f;
+  return fx_turn_at(f);
+}
+
+// (cos, sin) of an angle in radians, |ang| below 2^21: its significand times
+// 2^66 / (2 pi) (rounded: 2^-64 of the turns) as 128 bits, of which the fraction
+// of a turn is kept, 2^-43 of a radian at the largest angle and 2^-62 at one turn
+constexpr int kAngleBits = 21;
+__host__ __device__ __forceinline__ bool fx_angle_ok(double ang) {
+  return ((int)(dbits(ang) >> 52) & 0x7ff) < 1023 + kAngleBits;
+}
+__host__ __device__ __forceinline__ cpx<fx> fx_angle(double ang) {
+  constexpr unsigned long long kTurns = 11743562013128004906ULL;
+  const long long b = dbits(ang);
+  const int sh = 1077 - ((int)(b >> 52) & 0x7ff);  // 2^64 turns = significand kTurns >> sh
+  const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffULL) | (1ULL << 52), lo = m * kTurns;
+#ifdef __CUDA_ARCH__
+  const unsigned long long hi = __umul64hi(m, kTurns);
+#else
+  const unsigned long long hi = (unsigned long long)(((unsigned __int128)m * kTurns) >> 64);
+#endif
+  unsigned long long f = sh < 64 ? hi << (64 - sh) | lo >> sh : (sh < 128 ? hi >> (sh - 64) : 0);
+  if (b < 0) f = 0 - f;
+  return fx_turn_at(f);
 }
 
 // exp(2 pi i u (1 + rest 2^-83)); infinite and NaN u give NaN

@@ -240,6 +240,80 @@ __device__ __forceinline__ bool voxel_E_real(double beta, const VoxelInv& vi, do
   return false;
 }
 
+// Real solve in FP64 (real eps above beta^2, uniaxial or isotropic voxels) of
+// every beam of one voxel
+template <typename R, bool FOUR>
+__device__ __forceinline__ void voxel_op_real(const OpParams& p, const Grid& g, R* __restrict__ opv, int pix, int ray0,
+                                              int ray1) {
+  constexpr int nrec = FOUR ? OP_REC : REC_BLOCK;
+  const int HW = g.H * g.W;
+  const int y = pix / g.W, x = pix - y * g.W;
+  const long long eo = (p.layer + (int)blockIdx.z) * p.ev_s[0] + y * p.ev_s[1] + x * p.ev_s[2];
+  const long long ao = (p.layer + (int)blockIdx.z) * p.ea_s[0] + y * p.ea_s[1] + x * p.ea_s[2];
+  const size_t row = (size_t)y * g.W;
+  const int xs = p.permW ? p.permW[x] : x;
+  // the voxel's trigonometry and invariants, shared by every ray and window
+  double sa, ca;
+  sincos(p.epsa[ao + 2], &sa, &ca);
+  VoxelInv vi;
+  voxel_inv((const double*)p.epsv + eo, p.epsa[ao + 1], vi);
+  for (int rw = ray0 * p.nwin; rw < ray1 * p.nwin; ++rw) {
+    const double beta = p.wbeta[rw];
+    const double cp = p.wcos[rw], sp = p.wsin[rw];
+    // cos / sin of (azimuth - phi) by the angle-difference identities
+    const double cf = ca * cp + sa * sp, sf = sa * cp - ca * sp;
+    const double aw = p.uncorrected ? 0.0 : p.waw[rw];
+    double ev02, evs, c2;
+    if (p.wev02 != nullptr) {
+      ev02 = p.wev02[rw];
+      evs = p.wevs[rw];
+      c2 = p.wc2[rw];
+    } else {
+      ev02 = vi.ev[0] - beta * beta;
+      evs = sqrt(ev02);
+      c2 = vi.ev[0] * (ev02 + (vi.ev[2] - vi.ev[0]));
+    }
+    double E[2][4], al[4];
+    bool zero = voxel_E_real<FOUR>(beta, vi, ev02, evs, c2, sf, cf, E, al);
+    // back to the lab frame: rotate the E rows by the beam azimuth phi
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      if (!FOUR && (m & 1)) continue;
+      const double ex = E[0][m], ey = E[1][m];
+      E[0][m] = ex * cp - ey * sp;
+      E[1][m] = ex * sp + ey * cp;
+    }
+    const double detf = E[0][0] * E[1][2] - E[0][2] * E[1][0];
+    double detb = 1.0;
+    if (FOUR) detb = E[0][1] * E[1][3] - E[0][3] * E[1][1];
+    if (detf == 0.0 || detb == 0.0) zero = true;
+    // records in the bulk precision, the first column times scale / det
+    R rec[nrec];
+    if (zero) {
+#pragma unroll
+      for (int i = 0; i < nrec; ++i) rec[i] = (R)0;
+    } else {
+      const double sfd = p.scale / detf;
+      rec[0] = to_r<R>(E[0][0] * sfd); rec[1] = to_r<R>(E[0][2]); rec[2] = to_r<R>(E[1][0] * sfd); rec[3] = to_r<R>(E[1][2]);
+      rec[4] = to_r<R>((al[0] - aw) * p.d);
+      rec[5] = to_r<R>((al[2] - aw) * p.d);
+      if (FOUR) {
+        const double sbd = p.scale / detb;
+        rec[6] = to_r<R>(E[0][1] * sbd); rec[7] = to_r<R>(E[0][3]); rec[8] = to_r<R>(E[1][1] * sbd); rec[9] = to_r<R>(E[1][3]);
+        rec[10] = to_r<R>((al[1] + aw) * p.d);
+        rec[11] = to_r<R>((al[3] + aw) * p.d);
+      }
+    }
+    store_planes<nrec, R>(opv + ((size_t)rw * HW + row) * nrec, g.W, xs, rec);
+  }
+}
+
+// the same out of line, for the few complex64 voxels that the pair solve does not take
+template <bool FOUR>
+__device__ __noinline__ void voxel_op_wide(OpParams p, Grid g, float* opv, int pix, int ray0, int ray1) {
+  voxel_op_real<float, FOUR>(p, g, opv, pix, ray0, ray1);
+}
+
 // Lean solve for complex64 records (real eps above beta^2, uniaxial or
 // isotropic voxels) in pairs of FP32 numbers (48 bits, dtmm_common.cuh).  FP64
 // issues at 1/64 of the FP32 rate here: the same eigenvalues at 12 FP64
@@ -264,11 +338,20 @@ constexpr int kLeanChunk = 32;  // windows per shared-memory chunk (<= the block
 
 // cos and sin of an angle as pairs
 __device__ __forceinline__ void ff_sincos(double ang, ff& s, ff& c) {
-  const double u = ang * 0.15915494309189533577;
-  const cpx<fx> t = fx_turn(u);
+  const cpx<fx> t = fx_angle(ang);
   s = ff_q62(t.im.v);
   c = ff_q62(t.re.v);
-  if ((fx_hiword(u) & 0x7ff00000) == 0x7ff00000) s.h = c.h = __int_as_float(0x7fc00000);
+}
+
+// The pairs have the exponent range of FP32, and products of three eps occur:
+// values from 2^-30 to 2^30 (layers below 2^60 pixels) leave every term and its
+// low part inside it.  Voxels beyond that, and angles that fx_angle does not
+// take (2^21 rad, infinities), take the FP64 solve.
+__device__ __forceinline__ bool lean_range(double x) {
+  return (unsigned)(((int)(__double_as_longlong(x) >> 52) & 0x7ff) - 993) < 60u;
+}
+__device__ __forceinline__ bool lean_d(double x) {
+  return ((int)(__double_as_longlong(x) >> 52) & 0x7ff) < 1083;
 }
 
 template <bool FOUR>
@@ -278,7 +361,7 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
   constexpr int nrec = FOUR ? OP_REC : REC_BLOCK;
   const float scf = f32_rn(p.scale);
   const int HW = g.H * g.W;
-  const bool active = pix < HW;
+  bool active = pix < HW, wide = false;
   const bool uni = p.wev02 != nullptr;
   // the voxel's invariants, shared by every ray and window
   const ff z = ff_mk(0.0f, 0.0f);
@@ -296,8 +379,12 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
     const double* e = (const double*)p.epsv + eo;
     const double eo0 = e[0], ee = e[2], eps = p.uncorrected ? 0.0 : p.eps_dev[0];
     iso = eo0 == e[1] && e[1] == ee;
-    ff_sincos(p.epsa[ao + 1], vx.st, vx.ct);
-    ff_sincos(p.epsa[ao + 2], vx.sa, vx.ca);
+    const double theta = p.epsa[ao + 1], azim = p.epsa[ao + 2];
+    wide = !(lean_range(eo0) && lean_range(ee) && (p.uncorrected || lean_range(eps)) && lean_d(p.d) &&
+             fx_angle_ok(theta) && fx_angle_ok(azim));
+    active = !wide;
+    ff_sincos(theta, vx.st, vx.ct);
+    ff_sincos(azim, vx.sa, vx.ca);
     e0 = ff_of(eo0);
     e2 = ff_of(ee);
     n0 = ff_of(eo0 - eps);
@@ -417,6 +504,16 @@ __device__ __forceinline__ void voxel_op_lean(const OpParams& p, const Grid& g, 
       store_planes<nrec, float>(opv + ((size_t)(c0 + k) * HW + row) * nrec, g.W, xs, rec);
     }
   }
+  if (wide) voxel_op_wide<FOUR>(p, g, opv, pix, ray0, ray1);
+}
+
+// complex64 records of real eps; as many 128-thread blocks a SM as the pair solve
+// alone allows
+template <bool FOUR>
+__global__ void __launch_bounds__(128, FOUR ? 6 : 7) k_voxel_op_lean(OpParams p, Grid g, void* __restrict__ opv) {
+  const int ray0 = blockIdx.y * p.rays_per_thread;
+  voxel_op_lean<FOUR>(p, g, (float*)((unsigned char*)opv + (size_t)blockIdx.z * p.layer_bytes),
+                      blockIdx.x * blockDim.x + threadIdx.x, ray0, min(ray0 + p.rays_per_thread, p.nray));
 }
 
 // BIAX: the material holds biaxial voxels, which take the general
@@ -429,10 +526,6 @@ __global__ void k_voxel_op(OpParams p, Grid g, void* __restrict__ opv) {
   const int pix = blockIdx.x * blockDim.x + threadIdx.x;
   const int ray0 = blockIdx.y * p.rays_per_thread;
   const int ray1 = min(ray0 + p.rays_per_thread, p.nray);
-  if constexpr (REAL && sizeof(R) == 4) {  // every thread of the block: the solve shares window tables
-    voxel_op_lean<FOUR>(p, g, (float*)opv, pix, ray0, ray1);
-    return;
-  }
   if (pix >= HW) return;
   const int y = pix / g.W, x = pix - y * g.W;
   const long long eo = (p.layer + (int)blockIdx.z) * p.ev_s[0] + y * p.ev_s[1] + x * p.ev_s[2];
@@ -442,63 +535,13 @@ __global__ void k_voxel_op(OpParams p, Grid g, void* __restrict__ opv) {
   constexpr int nrec = FOUR ? OP_REC : REC_BLOCK;
   const size_t row = (size_t)y * g.W;
   const int xs = p.permW ? p.permW[x] : x;
-  // the voxel's trigonometry and invariants, shared by every ray and window
-  double sa, ca;
-  sincos(azim, &sa, &ca);
   if constexpr (REAL) {
-    VoxelInv vi;
-    voxel_inv((const double*)p.epsv + eo, theta, vi);
-    for (int rw = ray0 * p.nwin; rw < ray1 * p.nwin; ++rw) {
-      const double beta = p.wbeta[rw];
-      const double cp = p.wcos[rw], sp = p.wsin[rw];
-      // cos / sin of (azimuth - phi) by the angle-difference identities
-      const double cf = ca * cp + sa * sp, sf = sa * cp - ca * sp;
-      const double aw = p.uncorrected ? 0.0 : p.waw[rw];
-      double ev02, evs, c2;
-      if (p.wev02 != nullptr) {
-        ev02 = p.wev02[rw];
-        evs = p.wevs[rw];
-        c2 = p.wc2[rw];
-      } else {
-        ev02 = vi.ev[0] - beta * beta;
-        evs = sqrt(ev02);
-        c2 = vi.ev[0] * (ev02 + (vi.ev[2] - vi.ev[0]));
-      }
-      double E[2][4], al[4];
-      bool zero = voxel_E_real<FOUR>(beta, vi, ev02, evs, c2, sf, cf, E, al);
-      // back to the lab frame: rotate the E rows by the beam azimuth phi
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        if (!FOUR && (m & 1)) continue;
-        const double ex = E[0][m], ey = E[1][m];
-        E[0][m] = ex * cp - ey * sp;
-        E[1][m] = ex * sp + ey * cp;
-      }
-      const double detf = E[0][0] * E[1][2] - E[0][2] * E[1][0];
-      double detb = 1.0;
-      if (FOUR) detb = E[0][1] * E[1][3] - E[0][3] * E[1][1];
-      if (detf == 0.0 || detb == 0.0) zero = true;
-      // records in the bulk precision, the first column times scale / det
-      R rec[nrec];
-      if (zero) {
-#pragma unroll
-        for (int i = 0; i < nrec; ++i) rec[i] = (R)0;
-      } else {
-        const double sfd = p.scale / detf;
-        rec[0] = to_r<R>(E[0][0] * sfd); rec[1] = to_r<R>(E[0][2]); rec[2] = to_r<R>(E[1][0] * sfd); rec[3] = to_r<R>(E[1][2]);
-        rec[4] = to_r<R>((al[0] - aw) * p.d);
-        rec[5] = to_r<R>((al[2] - aw) * p.d);
-        if (FOUR) {
-          const double sbd = p.scale / detb;
-          rec[6] = to_r<R>(E[0][1] * sbd); rec[7] = to_r<R>(E[0][3]); rec[8] = to_r<R>(E[1][1] * sbd); rec[9] = to_r<R>(E[1][3]);
-          rec[10] = to_r<R>((al[1] + aw) * p.d);
-          rec[11] = to_r<R>((al[3] + aw) * p.d);
-        }
-      }
-      store_planes<nrec, R>((R*)opv + ((size_t)rw * HW + row) * nrec, g.W, xs, rec);
-    }
+    voxel_op_real<R, FOUR>(p, g, (R*)opv, pix, ray0, ray1);
     return;
   }
+  // the voxel's trigonometry, shared by every ray and window
+  double sa, ca;
+  sincos(azim, &sa, &ca);
   double st, ct;
   sincos(theta, &st, &ct);
   for (int rw = ray0 * p.nwin; rw < ray1 * p.nwin; ++rw) {
