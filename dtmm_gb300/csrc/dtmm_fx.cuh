@@ -287,7 +287,7 @@ __host__ __device__ __forceinline__ cpx<fx> fx_turn_at(unsigned long long f) {
   const long long z = (fx(d, 0) * fx(d, 0)).v;           // d^2 2^74
   const int zh = (int)(z >> 27), dh = (int)(d >> 30);    // d^2 2^47, d 2^38
   const int z2 = (int)(madw(zh, zh, 0) >> 32);           // d^4 2^62
-  const long long cm = (z >> 7) - (madw(z2, 43691, 0) >> 14);  // (1 - cos d) 2^68
+  const long long cm = (z >> 7) - (madw(z2, 715827883, 0) >> 28);  // (1 - cos d) 2^68 (2^28 64 / 24)
   const int q = zh - (int)(madw(z2 >> 15, 3277, 0) >> 16);     // (d^2 - d^4 / 20) 2^47
   const long long w = madw(dh, q, 0);                          // (d^3 - d^5 / 20) 2^85
   const long long sn = d - (madw((int)(w >> 29), 715827883, 0) >> 20);  // sin d 2^68
