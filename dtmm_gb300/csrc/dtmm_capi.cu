@@ -857,6 +857,10 @@ struct Engine {
     p.groups_inner = rec_bytes > ((size_t)64 << 20) ? 1 : 0;
     rl.lim = std::max(0, std::min(blim_max, d.width));
     rl.grid = p.groups_inner ? dim3(d.nray * ngrp * npg, d.height) : dim3(d.height, d.nray * ngrp * npg);
+    // few short lines: a thread per pixel for the operators (up to 128), where the
+    // blocks, two or three of 128 threads a SM, stay one wave
+    if (rl.grid.x * rl.grid.y <= (ls.maxl <= 16 ? 456 : 304))
+      rl.threads = std::max(rl.threads, std::min(std::min(128, most), d.width / 32 * 32));
     rl.pdl = pdl_for(rl.grid);
     mark(PROF_ROW);
     const cudaError_t e = sizeof(R) == 8 ? row_line(C, re, rl, p, g, Ub, Xb) : row_linef(C, re, rl, p, g, Ub, Xb);
