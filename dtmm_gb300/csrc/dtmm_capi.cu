@@ -477,6 +477,22 @@ cudaError_t launch_rows_line(const LineShape& ls, const void* src, void* dst, in
   return rows_line(L, src, dst, nlines, W, inv, tw, scale, lpb);
 }
 
+// Plain transforms (no band, no operators: real-space steps, refocusing) whose line kernels
+// lose to the shared-memory passes.  Refocusing, lines against shared memory, 1 / 6 / 18
+// images: complex128 162 points .91 / 1.16 / 1.19, 189 .82 / 1.21 / 1.13, 243 .82 / 1.46 / 1.51, own
+// columns 125 .86 / .96 / 1.43 and 512 (32 points a thread) 1.34 / 1.18 (but 200 .8, 250 .7 / 1.0, 500 .9);
+// complex64 189 .83 / 1.06 / 1.14, 243 .77 / 1.2 / 1.28, own 125 .84 / .94 / 1.32, 175 .91 / 1.12 / 1.32.
+template <typename R>
+bool line_plain_loses(int n, int images) {
+  const LineShape s = line_shape(n);
+  if (s.n2 <= 16 || n % 11 == 0) return false;
+  if (sizeof(R) == 8) {
+    if (line_side(s.n1, s.n2)) return s.n2 == 32 || (images >= 18 && s.n2 >= 5 * s.n1);
+    return images >= 6 && s.n2 >= 2 * s.n1;
+  }
+  return linef_side(s.n1, s.n2) ? images >= 18 && 2 * s.n2 >= 5 * s.n1 : images >= 6 && s.n2 > 2 * s.n1;
+}
+
 template <typename R>
 struct Engine {
   Prof* prof = nullptr;
@@ -579,9 +595,63 @@ struct Engine {
   bool pdl_sweep = false;
   bool pdl_for(dim3 grid) const { return pdl_sweep && prof == nullptr && (size_t)grid.x * grid.y <= 1216; }
 
-  // the line kernels take this side (fft_schedule 2 and 3 ask for the shared-memory passes)
-  bool line_on(int n) const { return d.fft_schedule <= 1 && line_shape(n).maxl > 0; }
-  bool row_line_on() const { return !row_reg() && line_on(d.width); }
+  // The line kernels take the rows / columns (set by setup).  fft_schedule 2 and 3 ask for the
+  // shared-memory passes, 1 for lines wherever a side splits; 0 leaves out the sides whose lines lose.
+  bool lineW = false, lineH = false;
+  bool row_line_on() const { return !row_reg() && lineW; }
+
+  // Rows and columns of one sweep whose two steps are so uneven that the shared-memory
+  // passes are faster: a step runs max(n1, n2) threads a line, of which one step uses n1, and
+  // lengths without kernels of their own spill from 18 points on.  It shows where few lines
+  // wait on a step's latency and where many fill the chip, less between.  Four layers, lines
+  // against shared memory (complex128 unless said; 2x2 method with 1 / 6 / 18 images):
+  //   nothing cut (pixels of 220 nm): 162 points 1.17 / 1.26 / 1.19, 189 1.15 / 1.20 / 1.15, 243 1.24 /
+  //     1.44 / 1.44, own kernels 125 1.07 / .99 / 1.23 (but 200 .94 / .80 / .80, 384 .95 / .84; 350
+  //     with complex records .91 / .93); complex64 189 1.02 / 1.08 / 1.11, 243 .98 / 1.10 / 1.10,
+  //     own 125 .87 / .92 / 1.09 (4x4 method .83 / .97 / 1.26)
+  //   cut at betamax (lines leave out what lies beyond): 162 1.11 / 1.01 / .90, 189 1.03 / .97 / .83, 243
+  //     1.20 / 1.17 / 1.02; own kernels with windows 125 1.33 / .73 / .91, 175 1.17 / .76 / .69; complex
+  //     records 125 1.08 / 1.04 / 1.18, with windows 162 1.10 / .94 / 1.08
+  // Sides with a factor 11 (a long shared-memory pass) keep the lines: 198 points .76 / .74 / .62.
+  bool line_loses(int n, bool cut) const {
+    const LineShape s = line_shape(n);
+    if (s.n2 <= 16 || n % 11 == 0) return false;
+    const bool dbl = sizeof(R) == 8, real = real_ops(), win = L.nwin > 1;
+    const bool own = real && (dbl ? line_side(s.n1, s.n2) : linef_side(s.n1, s.n2));
+    const bool u2 = s.n2 > 2 * s.n1, u3 = s.n2 >= 3 * s.n1, u5 = s.n2 >= 5 * s.n1;
+    const bool threes = n % 5 && n % 7 && 2 * s.n2 >= 3 * s.n1;  // short shared-memory passes
+    const int lines = NI * L.C;
+    if (!dbl) {
+      if (cut) return !own && u5 && lines >= 36;
+      return own ? u3 && lines >= 36 : u2 && lines >= 12;
+    }
+    if (own) return cut ? win && u3 && lines <= (u5 ? 4 : 2) : u5 && (lines <= 4 || lines >= 24);
+    if (n >= 256) return false;
+    if (!cut) return threes || (u2 && (real || lines <= 2 || lines >= 12));
+    if (u5) return lines <= 4 || lines >= 24;
+    if (u3 && n % 7) return (lines <= 2 || lines >= 12) && (!real || L.C == 2);
+    if (lines <= 2) return n % 5 && 2 * s.n2 >= 3 * s.n1;
+    return !real && win && threes && (lines <= 8 || lines >= 24);
+  }
+  // true if the axis of n points holds frequencies beyond the band limit
+  static bool axis_cut(int n, int lim) { return 2 * (long long)lim + 1 <= n - n / 10; }
+
+  // after the band limits are known
+  void choose_lines() {
+    const bool asked = d.fft_schedule <= 1;
+    lineW = asked && line_shape(d.width).maxl > 0;
+    lineH = asked && line_shape(d.height).maxl > 0;
+    if (d.fft_schedule != 0) return;
+    if (L.op_one == 0) {  // real-space steps: plain transforms, whole grids
+      lineW = lineW && !line_plain_loses<R>(d.width, NI);
+      lineH = lineH && !line_plain_loses<R>(d.height, NI);
+    } else if (lineW && lineH && line_loses(d.width, axis_cut(d.width, blim_max)) &&
+               line_loses(d.height, axis_cut(d.height, blimH_max))) {
+      lineW = lineH = false;
+    } else if (!axis_cut(d.height, blimH_max)) {
+      lineH = lineH && !line_plain_loses<R>(d.height, NI);
+    }
+  }
 
   // the buffer that holds a row pass's band-limited output, if any
   const cpx<R>* row_out = nullptr;
@@ -603,7 +673,7 @@ struct Engine {
         return DTMM_OK;
       }
     }
-    if (line_on(d.width)) {
+    if (lineW) {
       const cudaError_t e = launch_rows_line<R>(line_shape(d.width), data, data, nlines, d.width, inv, P(L.twW), scale, st);
       ++launches;
       if (e != cudaSuccess) return fail(DTMM_ECUDA, "launch k_rows_line: %s", cudaGetErrorString(e));
@@ -724,7 +794,7 @@ struct Engine {
     const int cm = cin > cout ? cin : cout;
     if (col_reg()) return launch_col_reg(p, in, out);
     // (after shared-memory row passes the out-of-band columns have to be written)
-    if (line_on(d.height) && p.band_skip == 2) return launch_col_line(p, in, out);
+    if (lineH && (p.band_skip == 2 || kop != KOP_DIAG)) return launch_col_line(p, in, out);
     p.tc = tile_cols(cm, true);
     const size_t smem = 2 * (size_t)cm * d.height * p.tc * sizeof(cpx<R>) + d.height * (sizeof(cpx<R>) + sizeof(int));
     CK(cudaFuncSetAttribute(k_layer_col<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1372,6 +1442,7 @@ struct Engine {
         CKL("k_set_scalars");
       }
     }
+    choose_lines();
     // FFT tables
     k_fft_tables<R><<<(d.height + 255) / 256, 256, 0, st>>>(pH, P(L.twH), A<int>(L.permH));
     CKL("k_fft_tables");
@@ -2522,7 +2593,9 @@ int diffract_impl(int H, int W, int nimg, int nlam, const void* dmat, const void
   int lpb = std::max(1, std::min(16, 4096 / W));
   size_t smem = (size_t)lpb * W * sizeof(cpx<R>) + W * (sizeof(cpx<R>) + sizeof(int));
   if (smem > 220 * 1024) return fail(DTMM_ENOTSUP, "row of %d pixels too large for one block", W);
-  const LineShape lsW = line_shape(W), lsH = line_shape(H);
+  const LineShape none{0, 0, 0};
+  const LineShape lsW = line_plain_loses<R>(W, nimg) ? none : line_shape(W);
+  const LineShape lsH = line_plain_loses<R>(H, nimg) ? none : line_shape(H);
   if (rrows) {
     const cudaError_t e = fft_rows_reg_dispatch(W, false, rl, in, X, nlines, twW, 1.0f);
     ++launches;

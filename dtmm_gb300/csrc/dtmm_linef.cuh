@@ -416,6 +416,13 @@ __global__ void __launch_bounds__(256, linef_col_blocks(MAXL, CN1))
   X(5, 9) X(5, 10) X(5, 15) X(5, 25) X(6, 8) X(6, 10) X(7, 9) X(7, 25) X(8, 9) X(9, 10) X(9, 15) X(10, 10) \
   X(10, 11) X(10, 12) X(10, 14) X(10, 15) X(10, 20) X(10, 25) X(11, 20) X(12, 14) X(12, 15) X(14, 14) X(14, 15) \
   X(14, 20) X(14, 25) X(15, 15) X(15, 18) X(15, 20) X(15, 22) X(16, 22) X(18, 20)
+inline bool linef_side(int n1, int n2) {
+#define DTMM_LINEF_IS(A, B) \
+  if (n1 == A && n2 == B) return true;
+  DTMM_LINEF_SIDES(DTMM_LINEF_IS)
+#undef DTMM_LINEF_IS
+  return false;
+}
 #define DTMM_LINEF_DECLARE(A, B)                                                                                     \
   cudaError_t row_linef_##A##_##B(int C, const LineLaunch& L, const RowParams& p, const Grid& g, const void* U, void* X); \
   cudaError_t col_linef_##A##_##B(const LineLaunch& L, const ColParams& p, const Grid& g, const void* in, void* out);

@@ -508,7 +508,8 @@ class DevicePlan:
         (results are bit-identical); ``fft_schedule`` 1/2/3 selects the
         two-step transforms in registers (sides that do not split take shared
         memory), radix-4-first or radix-8-first shared memory passes (results
-        agree to rounding).
+        agree to rounding); 0 takes the first two, whichever the engine's
+        rule finds the faster.
         """
         self.desc.fft_schedule = int(fft_schedule)
         self.desc.row_group = int(row_group)

@@ -84,7 +84,8 @@ typedef struct dtmm_transfer_desc {
   int real_path;
   /* tuning (0 = built-in choice; results do not depend on row_group and
      col_tile): wavelengths per row block, columns per column block, and the
-     line transform schedule: 1 = two-step transforms in registers, 2 = shared-memory
+     line transform schedule: 0 = two-step transforms in registers where they are the
+     faster ones, 1 = wherever a side splits, 2 = shared-memory
      mixed radix with radix-4 passes first, 3 = the same with radix-8 first */
   int row_group;
   int col_tile;
