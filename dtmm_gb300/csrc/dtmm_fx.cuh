@@ -212,14 +212,13 @@ __host__ __device__ __forceinline__ cpx<fx> fx_shift(cpx<fx> a, int r) {
 // x in the fixed point of a line whose largest biased exponent is emax, with
 // g guard bits: x 2^(1082 - g - emax) rounded to nearest, below 2^(60 - g);
 // integer operations (the hardware conversion issues at the FP64 rate).
-// Subnormal x count as zero (2^-1022 of range below the largest entry, or a
-// line of subnormals).
+// Subnormal x: the exponent of the smallest normal number, no leading one.
 __host__ __device__ __forceinline__ fx to_fx(double x, int emax, int g) {
   const long long b = dbits(x);
   const int e = (int)(b >> 52) & 0x7ff;
-  const int r = g + 2 + emax - e;  // right shift of the 63-bit significand, less one
-  const unsigned long long m = ((unsigned long long)b << 10 | (1ULL << 62)) & 0x7fffffffffffffffULL;
-  long long t = (e == 0 || r > 62) ? 0 : (long long)(m >> (r & 63));
+  const int r = g + 2 + emax - (e != 0 ? e : 1);  // right shift of the 63-bit significand, less one
+  const unsigned long long m = ((unsigned long long)b << 10 & 0x3fffffffffffffffULL) | (e != 0 ? 1ULL << 62 : 0ULL);
+  long long t = r > 62 ? 0 : (long long)(m >> (r & 63));
   t = (t + 1) >> 1;
   return fx(b < 0 ? -t : t, 0);
 }
