@@ -6,7 +6,7 @@ Workload (the precision configuration of the reference's benchmark set):
 256 x 256 grid, 60 layers of 1 pixel, 50 nm pixels, 9 wavelengths
 380-780 nm, x and y polarisations at normal incidence, seeded twisted nematic
 (no 1.52, ne 1.71, 8-mode perturbation of amplitude 0.3 rad), complex64 bulk
-with the eigen-solve in FP32 pairs (48 bits).  One step = one whole transfer_field of that
+with the eigen-solve in FP32 pairs (about 45 bits).  One step = one whole transfer_field of that
 workload; the unit is voxel x wavelength updates (H*W*layers*lambdas*
 polarisations*passes = 2.12e8 per step).
 
@@ -46,7 +46,7 @@ OPTS = dict(method="4x4", diffraction=3, npass=3, beta=0.0, phi=0.0)
 BYTES_PER_UPDATE = 2 * 4 * 8 + 48.0 / (len(WAVELENGTHS) * 2)
 CONFIG = {
     "workload": "transfer_field 4x4 npass=3 diffraction=3, 256x256 grid, 60 layers, 9 wavelengths 380-780 nm, "
-                "x+y polarisation, twisted nematic (no 1.52, ne 1.71, amp 0.3), complex64 bulk, eigen-solve in FP32 pairs (48 bits)",
+                "x+y polarisation, twisted nematic (no 1.52, ne 1.71, amp 0.3), complex64 bulk, eigen-solve in FP32 pairs (about 45 bits)",
     "grid": "256x256", "layers": 60, "wavelengths": 9, "polarisations": 2, "passes": 3, "windows": 9,
     "l2": "flushed between timed steps (256 MiB write)",
 }
@@ -283,7 +283,7 @@ def run_batch(args, dev, ninst=48, seed=0):
                                "graph; grids log-uniform 64-512 rounded to 7-smooth multiples of 16, 20-120 "
                                "layers, 1-9 wavelengths in 400-700 nm, 7 rays (beta 0, +-0.1, +-0.2 at phi 0; "
                                "+-0.1 at phi 90 deg), x+y polarisation, twisted nematic (no 1.5, ne 1.7, amp 0.2), "
-                               "complex64 bulk, eigen-solve in FP32 pairs (48 bits), autotuned launch shapes" % ninst,
+                               "complex64 bulk, eigen-solve in FP32 pairs (about 45 bits), autotuned launch shapes" % ninst,
                    "instances": ninst, "streams": args.streams,
                    "l2": "inputs larger than L2 (%.1f GB of input fields)" % (in_bytes / 1e9)},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
@@ -393,7 +393,7 @@ def run_2x2(args, dev):
         "vs_baseline": None, "dtype": "c64", "data": "synthetic",
         "config": {"workload": "transfer_field 2x2, diffraction 5 (25 windows), no reflection, 1024x1024 grid, "
                                "%d layers, 100 nm pixels, wavelengths 450/550/650 nm, x+y polarisation, in-plane "
-                               "nematic (16-mode azimuth, ne 1.6, no 1.5), complex64 bulk, eigen-solve in FP32 pairs (48 bits)" % nl,
+                               "nematic (16-mode azimuth, ne 1.6, no 1.5), complex64 bulk, eigen-solve in FP32 pairs (about 45 bits)" % nl,
                    "l2": "flushed between timed steps (256 MiB write); fields (100 MB) are near L2 size"},
         "roofline": {"bound": "hbm", "achieved": achieved_row, "peak": peak, "unit": "GB/s",
                      "frac": achieved_row / peak, "traffic": None, "peak_source": peak_kind,
@@ -636,7 +636,7 @@ def run_serve(args, dev):
         "config": {"workload": "serving: Poisson stream of %d POM simulation requests at %g req/s, each a 4x4 "
                                "transfer_field (diffraction 1, npass 1, normal incidence, x+y polarisation) and its "
                                "crossed-polarizer sRGB image, grids log-uniform 64-512, 20-120 layers, 1-9 "
-                               "wavelengths, twisted nematic built on the device, complex64 bulk, eigen-solve in FP32 pairs (48 bits); "
+                               "wavelengths, twisted nematic built on the device, complex64 bulk, eigen-solve in FP32 pairs (about 45 bits); "
                                "continuous batching over %d stream slots, %g GB HBM admission budget"
                                % (args.requests, args.rate, args.slots, args.hbm_budget / 1e9),
                    "requests": args.requests, "rate": args.rate, "slots": args.slots,

@@ -715,7 +715,7 @@ struct Engine {
     } else {
       const int cm = std::max(p.cin, p.cout);
       int tx = kColLines / cm;
-      if (d.col_tile > 0) tx = std::min(tx, d.col_tile);
+      if (d.col_tile > 0) tx = std::min(tx, d.col_tile);  // (wider tiles exceed the block)
       p.tc = tx = std::min(tx, d.width);
       RegLaunch rl = col_reg_shape(d.height, cm * tx, st);
       rl.grid = dim3(band_tiles(p, tx), NI);
@@ -2037,8 +2037,7 @@ struct Engine {
     return launch_rows(f, 4, true, 1.0 / d.width);
   }
 
-  // byte offset of the backward-mode records in a voxel's operator records
-  // the backward blocks' planes of a row of records
+  // byte offset of the backward blocks' planes in a row of records
   size_t back_records() const { return (size_t)REC_BLOCK * d.width * (real_ops() ? sizeof(R) : sizeof(cpx<R>)); }
 
   // 2x2 method in k-space (reflection 0 or 1; dtmm/propagate_2x2.py:19-87,

@@ -136,9 +136,10 @@ __host__ __device__ __forceinline__ double f64_of(float f) {
 
 // ---------------------------------------------------------------------------
 // Pairs of FP32 numbers, h + l with |l| a few last places of h at most: about
-// 46 bits at FP32 rates (Dekker, "A floating-point technique for extending the
+// 45 bits a step at FP32 rates (Dekker, "A floating-point technique for extending the
 // available precision", 1971; products by FMA).  Every sum and product is
-// rounded on its own (no contraction).
+// rounded on its own (no contraction); results are not normalised, so a sum's
+// error is relative to its operands, not to what a cancellation leaves.
 // ---------------------------------------------------------------------------
 struct ff {
   float h, l;
@@ -199,11 +200,6 @@ __host__ __device__ __forceinline__ ff ff_q62(long long v) {
   const int lo = (int)((v - ((long long)hi << 38)) >> 7);
   return ff_mk((float)hi * 5.9604644775390625e-8f, (float)lo * 2.7755575615628914e-17f);  // 2^-24, 2^-55
 }
-
-#ifdef __CUDACC__
-// d == 0 (either sign), in integer arithmetic
-__device__ __forceinline__ bool is_zero_d(double d) { return (__double_as_longlong(d) << 1) == 0; }
-#endif
 
 __device__ __forceinline__ cpx<double> cvt_d(cpx<float> a) { return mk<double>(a.re, a.im); }
 __device__ __forceinline__ cpx<double> cvt_d(cpx<double> a) { return a; }

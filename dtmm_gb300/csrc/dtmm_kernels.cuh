@@ -315,7 +315,7 @@ __device__ __noinline__ void voxel_op_wide(OpParams p, Grid g, float* opv, int p
 }
 
 // Lean solve for complex64 records (real eps above beta^2, uniaxial or
-// isotropic voxels) in pairs of FP32 numbers (48 bits, dtmm_common.cuh).  FP64
+// isotropic voxels) in pairs of FP32 numbers (about 45 bits a step, dtmm_common.cuh).  FP64
 // issues at 1/64 of the FP32 rate here: the same eigenvalues at 12 FP64
 // operations a voxel and window kept that pipe 87 % busy and took 0.86 ms for
 // 1024 x 1024 voxels and 25 windows; a pair operation costs 4 to 8 FP32 ones.

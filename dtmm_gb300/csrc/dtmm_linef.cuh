@@ -3,7 +3,8 @@
 // n2 up to 32 (`line_shape`), two steps of register DFTs.  Slots, threads and
 // steps are those of dtmm_linekern.cuh, in FP32 arithmetic.  The sides of
 // DTMM_LINEF_SIDES have n1 and n2 at compile time: no switch over lengths, index
-// arithmetic by constants and no spills at fewer registers.
+// arithmetic by constants and no spills at fewer registers.  They are the sides of the
+// complex128 table (a choice, dtmm_linekern.cuh) up to 360 without a register transform.
 //
 // In shared-memory mixed-radix passes (prime by prime, every column of the
 // grid, the whole band) 330-point rows of 8 images took 114 us a layer and

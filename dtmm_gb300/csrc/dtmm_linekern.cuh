@@ -595,14 +595,17 @@ __global__ void __launch_bounds__(line_threads(MAXL, CN1), line_blocks(MAXL, CN1
 }
 
 // ---------------------------------------------------------------------------
-// Launch glue.  The sides of DTMM_LINE_SIDES (the most even splits n1 n2 of the
-// sides grids are usually chosen at, 45 to 1024) have row (real operator records) and
-// column kernels with n1 x n2 known at compile time, instantiated in
-// dtmm_line_<a..o>.cu: no switch and few spills, so that more blocks fit a SM.
+// Launch glue.  The sides of DTMM_LINE_SIDES have row (real operator records) and
+// column kernels with n1 x n2 (the most even split) known at compile time, instantiated
+// in dtmm_line_<a..o>.cu: no switch and few spills, so that more blocks fit a SM.  Which
+// sides these are is a choice, not a rule: multiples of 16 and of 5 and a few others from 45 to
+// 1024, those of the tests, the benchmark and perf/cases.py among them, 53 of the 135 in that
+// range that split, for the size of the library (2 MB a side).
 // Ten layers, run-time lengths -> these (row / column pass, ms): side 48, one window
 // .28 / .33 -> .21 / .24; 112, nine windows 6.9 / 1.24 -> 5.3 / .99; 200 14.4 / 3.2 ->
 // 6.6 / 1.6; 320 19.0 / 4.2 -> 11.3 / 2.1; 512 38.2 / 8.5 -> 32.3 / 6.5; 1024 199 / 29.7 ->
-// 170 / 24.0.  Every other side takes the run-time kernels of dtmm_line_any*.cu.
+// 170 / 24.0.  Every other side takes the run-time kernels of dtmm_line_any*.cu, or where
+// those lose (Engine::line_loses) the shared-memory passes.
 // ---------------------------------------------------------------------------
 struct LineLaunch {
   dim3 grid;

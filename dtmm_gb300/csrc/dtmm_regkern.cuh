@@ -36,12 +36,12 @@ __device__ __forceinline__ unsigned group_mask() {
   }
 }
 
-// row buffer stride (complex elements): with N1 = 4 or 8 several line groups
-// share a half-warp, and a stride of W + 4 (W + 8) puts their exchange slots
-// on disjoint banks; W is a multiple of 16 for every listed side
 // wavelengths per row block at most (the engine caps row_group here)
 constexpr int kMaxRowGroup = 64;
 
+// row buffer stride (complex elements): with N1 = 4 or 8 several line groups
+// share a half-warp, and a stride of W + 4 (W + 8) puts their exchange slots
+// on disjoint banks; W is a multiple of 16 for every listed side
 __host__ __device__ constexpr int reg_row_stride(int n1, int w) { return n1 == 4 ? w + 4 : (n1 == 8 ? w + 8 : w); }
 
 // Band variants of the row pass.  The window rows arrive band-limited: every

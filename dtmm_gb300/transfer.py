@@ -9,7 +9,7 @@ the transfer itself is one call into the CUDA library
 
 Extension: ``precision=`` selects the bulk arithmetic, "double" (complex128,
 the reference's precision, the default) or "mixed" (complex64 bulk; FP64
-k-space tables, the eigen-solve in FP64 or, for real eps, FP32 pairs of 48 bits); ``set_precision`` changes the default.
+k-space tables, the eigen-solve in FP64 or, for real eps, FP32 pairs of about 45 bits a step); ``set_precision`` changes the default.
 """
 from __future__ import annotations
 
@@ -44,7 +44,7 @@ _precision = ["double"]
 
 
 def set_precision(p):
-    """Default bulk precision: "double" (complex128) or "mixed" (complex64 bulk, FP64 or 48-bit eigen-solve)."""
+    """Default bulk precision: "double" (complex128) or "mixed" (complex64 bulk, eigen-solve in FP64 or FP32 pairs)."""
     if p not in ("double", "mixed"):
         raise ValueError("precision must be 'double' or 'mixed'")
     old = _precision[0]

@@ -37,7 +37,7 @@ extern "C" {
    (dtmm/propagate_4x4.py:515-560); 4x4, any reflection mode, any npass */
 #define DTMM_DIFFRACTION_FULL (-1)
 
-#define DTMM_PRECISION_MIXED 0  /* complex64 bulk, FP64 k-space tables, eigen-solve in FP64 or FP32 pairs (48 bits) */
+#define DTMM_PRECISION_MIXED 0  /* complex64 bulk, FP64 k-space tables, eigen-solve in FP64 or FP32 pairs (about 45 bits a step) */
 #define DTMM_PRECISION_DOUBLE 1 /* complex128 bulk (the reference's default precision), lines transformed in 64-bit block fixed point */
 
 typedef struct dtmm_transfer_desc {
