@@ -1151,21 +1151,26 @@ struct Engine {
         k_voxel_op_lean<true><<<grid, 128, 0, s>>>(p, g, op);
       else
         k_voxel_op_lean<false><<<grid, 128, 0, s>>>(p, g, op);
-    } else if (real_ops()) {
-      if (p.four)
-        k_voxel_op<double, true, true, false><<<grid, 128, 0, s>>>(p, g, op);
-      else
-        k_voxel_op<double, true, false, false><<<grid, 128, 0, s>>>(p, g, op);
     } else if (d.biaxial) {
       if (p.four)
-        k_voxel_op<R, false, true, true><<<grid, 128, 0, s>>>(p, g, op);
+        k_voxel_op<R, true, true><<<grid, 128, 0, s>>>(p, g, op);
       else
-        k_voxel_op<R, false, false, true><<<grid, 128, 0, s>>>(p, g, op);
+        k_voxel_op<R, false, true><<<grid, 128, 0, s>>>(p, g, op);
+    } else if constexpr (sizeof(R) == 4) {
+      if (p.four)
+        k_voxel_op<R, true, false><<<grid, 128, 0, s>>>(p, g, op);
+      else
+        k_voxel_op<R, false, false><<<grid, 128, 0, s>>>(p, g, op);
+    } else if (real_ops()) {
+      if (p.four)
+        k_voxel_op_c128<true, true><<<grid, 128, 0, s>>>(p, g, op);
+      else
+        k_voxel_op_c128<true, false><<<grid, 128, 0, s>>>(p, g, op);
     } else {
       if (p.four)
-        k_voxel_op<R, false, true, false><<<grid, 128, 0, s>>>(p, g, op);
+        k_voxel_op_c128<false, true><<<grid, 128, 0, s>>>(p, g, op);
       else
-        k_voxel_op<R, false, false, false><<<grid, 128, 0, s>>>(p, g, op);
+        k_voxel_op_c128<false, false><<<grid, 128, 0, s>>>(p, g, op);
     }
     mark_on(PROF_OP, s);
     CKL("k_voxel_op");
@@ -1624,7 +1629,10 @@ struct Engine {
   int feed_begin(int pass, const std::vector<int>& order, const std::vector<double>& ds, OpFeed& f) {
     f.ready.assign(order.size(), nullptr);
     if (L.cache_ops && pass > 0) return DTMM_OK;  // reused
-    if (st2 == nullptr) st2 = side_stream(st);
+    // (biaxial operators of complex64 transfers take longer than the passes, and longer still beside
+    // them: their 880 bytes of stack a thread lose L1 to the passes' shared memory.  121 x 80, nine
+    // windows, ten layers: 29.0 + 1.0 ms one after the other, 41 to 55 side by side)
+    if (st2 == nullptr) st2 = d.biaxial && sizeof(R) == 4 ? st : side_stream(st);
     if (st2 == nullptr) return DTMM_OK;
     int rc = wait_for(st2, st);  // inputs of the operators (setup, earlier passes)
     if (rc) return rc;

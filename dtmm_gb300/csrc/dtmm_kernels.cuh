@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(128, FOUR ? 6 : 7) k_voxel_op_lean(OpParams p,
 // eigen-solve (complex path only; without BIAX every voxel is isotropic or
 // uniaxial and the kernel keeps the registers of those closed forms)
 template <typename R, bool REAL, bool FOUR, bool BIAX>
-__global__ void k_voxel_op(OpParams p, Grid g, void* __restrict__ opv) {
+__device__ __forceinline__ void voxel_op_general(OpParams p, const Grid& g, void* __restrict__ opv) {
   const int HW = g.H * g.W;
   opv = (unsigned char*)opv + (size_t)blockIdx.z * p.layer_bytes;
   const int pix = blockIdx.x * blockDim.x + threadIdx.x;
@@ -661,6 +661,21 @@ __global__ void k_voxel_op(OpParams p, Grid g, void* __restrict__ opv) {
   }
   store_planes<nrec, cpx<R>>((cpx<R>*)opv + ((size_t)rw * HW + row) * nrec, g.W, xs, rec);
   }
+}
+
+template <typename R, bool FOUR, bool BIAX>
+__global__ void k_voxel_op(OpParams p, Grid g, void* __restrict__ opv) {
+  voxel_op_general<R, false, FOUR, BIAX>(p, g, opv);
+}
+
+// complex128 bulk, uniaxial or isotropic voxels.  The bounds hold the blocks a SM: at 86
+// registers instead of 80 (five blocks for six) the row passes beside the operators went
+// from 13.9 to 20.6 ms (2x2 method, absorbing voxels, 162 x 162, nine windows, 14 layers).
+// complex64 transfers, whose passes leave the FP64 pipe alone, lost 5 to 17 % by them.
+template <bool REAL, bool FOUR>
+__global__ void __launch_bounds__(128, REAL ? (FOUR ? 5 : 8) : (FOUR ? 3 : 6))
+    k_voxel_op_c128(OpParams p, Grid g, void* __restrict__ opv) {
+  voxel_op_general<double, REAL, FOUR, false>(p, g, opv);
 }
 
 // ---------------------------------------------------------------------------
@@ -2403,7 +2418,7 @@ __global__ void __launch_bounds__(256) k_layer_col(ColParams p, Grid g, const cp
 // slots q of the inverse transform's output (x = iperm[q]) and accumulates in
 // the same slots, the input order of the forward transform.  Operator records
 // are read once per block and window, phases once per wavelength.
-// REAL: records are real (see k_voxel_op).
+// REAL: records are real (see voxel_op_general).
 template <typename R, int C, bool REAL>
 __global__ void __launch_bounds__(256, 3) k_layer_row(RowParams p, Grid g, const cpx<R>* __restrict__ U,
                                                    cpx<R>* __restrict__ X) {
