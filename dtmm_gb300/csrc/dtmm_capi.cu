@@ -477,20 +477,29 @@ cudaError_t launch_rows_line(const LineShape& ls, const void* src, void* dst, in
   return rows_line(L, src, dst, nlines, W, inv, tw, scale, lpb);
 }
 
-// Plain transforms (no band, no operators: real-space steps, refocusing) whose line kernels
-// lose to the shared-memory passes.  Refocusing, lines against shared memory, 1 / 6 / 18
-// images: complex128 162 points .91 / 1.16 / 1.19, 189 .82 / 1.21 / 1.13, 243 .82 / 1.46 / 1.51, own
-// columns 125 .86 / .96 / 1.43 and 512 (32 points a thread) 1.34 / 1.18 (but 200 .8, 250 .7 / 1.0, 500 .9);
-// complex64 189 .83 / 1.06 / 1.14, 243 .77 / 1.2 / 1.28, own 125 .84 / .94 / 1.32, 175 .91 / 1.12 / 1.32.
+// Plain transforms (no band, no operators: real-space steps, refocusing, and columns of sweeps that the
+// band does not cut) whose line kernels lose to the shared-memory passes.  Refocusing 96-point columns
+// (rows) of n points, lines against shared memory, 1 / 6 / 18 images:
+//   rows: complex128 125 points .85 / 1.05 / 1.24, 243 .66 / .93 / 1.11 (but 162 .76 / .88 / .87, 250 .61 / .86 / .90);
+//     complex64 125 .86 / .90 / 1.22, 175 .81 / .83 / 1.14, 250 .71 / .84 / 1.11
+//   columns: complex128 without kernels of their own, n2 >= 1.5 n1: 162 1.08 / 1.18 / 1.15, 216 1.03 / 1.20 /
+//     1.08, 243 1.03 / 1.33 / 1.37; own: 125 .90 / 1.19 / 1.15, 512 (32 points a thread of 16) 1.22 / 1.16 / .98
+//     and on 512 x 512 grids 1.34 / 1.18 (but 250 .92 / 1.06 / .90, 640 .96 / .89 / .89, 1024 .95 / .78 / .76);
+//     complex64 162 .91 / .95 / 1.05, 243 .82 / .95 / 1.09
 template <typename R>
-bool line_plain_loses(int n, int images) {
+bool line_rows_lose(int n, int images) {
+  const LineShape s = line_shape(n);
+  if (s.n2 <= 16 || n % 11 == 0 || images < 18) return false;
+  if (sizeof(R) == 4) return 2 * s.n2 >= 5 * s.n1;
+  return s.n2 >= 5 * s.n1 || (n % 5 && n % 7 && s.n2 >= 3 * s.n1);
+}
+template <typename R>
+bool line_cols_lose(int n, int images) {
   const LineShape s = line_shape(n);
   if (s.n2 <= 16 || n % 11 == 0) return false;
-  if (sizeof(R) == 8) {
-    if (line_side(s.n1, s.n2)) return s.n2 == 32 || (images >= 18 && s.n2 >= 5 * s.n1);
-    return images >= 6 && s.n2 >= 2 * s.n1;
-  }
-  return linef_side(s.n1, s.n2) ? images >= 18 && 2 * s.n2 >= 5 * s.n1 : images >= 6 && s.n2 > 2 * s.n1;
+  if (sizeof(R) == 4) return images >= 18 && !linef_side(s.n1, s.n2) && reg_lanes(n) == 0 && s.n2 >= 2 * s.n1;
+  if (line_side(s.n1, s.n2)) return (s.n2 == 32 && s.n2 >= 2 * s.n1) || (images >= 6 && s.n2 >= 5 * s.n1);
+  return n < 256 && 2 * s.n2 >= 3 * s.n1;
 }
 
 template <typename R>
@@ -643,13 +652,13 @@ struct Engine {
     lineH = asked && line_shape(d.height).maxl > 0;
     if (d.fft_schedule != 0) return;
     if (L.op_one == 0) {  // real-space steps: plain transforms, whole grids
-      lineW = lineW && !line_plain_loses<R>(d.width, NI);
-      lineH = lineH && !line_plain_loses<R>(d.height, NI);
+      lineW = lineW && !line_rows_lose<R>(d.width, NI);
+      lineH = lineH && !line_cols_lose<R>(d.height, NI);
     } else if (lineW && lineH && line_loses(d.width, axis_cut(d.width, blim_max)) &&
                line_loses(d.height, axis_cut(d.height, blimH_max))) {
       lineW = lineH = false;
     } else if (!axis_cut(d.height, blimH_max)) {
-      lineH = lineH && !line_plain_loses<R>(d.height, NI);
+      lineH = lineH && !line_cols_lose<R>(d.height, NI);
     }
   }
 
@@ -2601,8 +2610,8 @@ int diffract_impl(int H, int W, int nimg, int nlam, const void* dmat, const void
   size_t smem = (size_t)lpb * W * sizeof(cpx<R>) + W * (sizeof(cpx<R>) + sizeof(int));
   if (smem > 220 * 1024) return fail(DTMM_ENOTSUP, "row of %d pixels too large for one block", W);
   const LineShape none{0, 0, 0};
-  const LineShape lsW = line_plain_loses<R>(W, nimg) ? none : line_shape(W);
-  const LineShape lsH = line_plain_loses<R>(H, nimg) ? none : line_shape(H);
+  const LineShape lsW = line_rows_lose<R>(W, nimg) ? none : line_shape(W);
+  const LineShape lsH = line_cols_lose<R>(H, nimg) ? none : line_shape(H);
   if (rrows) {
     const cudaError_t e = fft_rows_reg_dispatch(W, false, rl, in, X, nlines, twW, 1.0f);
     ++launches;

@@ -1,7 +1,7 @@
 """Sides whose two-step line transforms lose to the shared-memory passes take those (GPU).
 
 ``fft_schedule`` 0 is the engine's choice, 1 the lines wherever a side splits, 2 the shared-memory passes: the
-choice shows in the bits, and both agree to the bounds of ``test_gpu_line.py`` (2e-14 in complex128, 3e-6 in
+choice, for rows and columns together or for the columns alone, shows in the bits, and all agree to the bounds of ``test_gpu_line.py`` (2e-14 in complex128, 3e-6 in
 complex64; two layers here as there).
 """
 import numpy as np
@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 # (shape, precision, method, wavelengths, polarisations, diffraction, pixel size, betamax, absorbing, reflection, shared)
 CASES = [
     ((162, 162), "double", "4x4", 2, 1, 1, 220.0, 1.4, False, None, True),    # nothing cut
-    ((162, 160), "double", "4x4", 2, 1, 1, 220.0, 1.4, False, None, False),   # one side only
+    ((162, 160), "double", "4x4", 2, 1, 1, 220.0, 1.4, False, None, "columns"),  # one side only
     ((125, 125), "double", "4x4", 1, 1, 3, 220.0, 1.4, False, None, True),
     ((125, 125), "double", "4x4", 2, 1, 3, 220.0, 1.4, False, None, False),   # neither few nor many lines
     ((198, 198), "double", "4x4", 2, 1, 1, 220.0, 1.4, False, None, False),   # a factor 11
@@ -26,8 +26,9 @@ CASES = [
     ((125, 125), "double", "4x4", 3, 2, 1, 100.0, 0.8, True, None, True),     # complex records
     ((162, 162), "double", "4x4", 2, 1, 3, 100.0, 0.8, True, None, True),
     ((160, 160), "double", "4x4", 2, 1, 3, 100.0, 0.8, True, None, False),
-    ((162, 162), "double", "4x4", 3, 2, 1, 100.0, 0.8, False, 2, True),       # real-space steps
-    ((162, 162), "double", "4x4", 1, 1, 1, 100.0, 0.8, False, 2, False),
+    ((162, 162), "double", "4x4", 3, 2, 1, 100.0, 0.8, False, 2, "columns"),  # real-space steps
+    ((243, 160), "double", "2x2", 1, 1, 1, 100.0, 0.8, False, 2, "columns"),
+    ((160, 162), "double", "4x4", 1, 1, 1, 100.0, 0.8, False, 2, False),
 ]
 
 
@@ -56,13 +57,14 @@ def test_choice_of_the_line_passes(case):
         plan.run(fin.clone(), o)
         out.append(o)
     auto, lines, passes = out
-    assert torch.equal(auto, passes if shared else lines)
+    assert torch.equal(auto, lines) == (shared is False) and torch.equal(auto, passes) == (shared is True)
     assert not torch.equal(lines, passes)
     tol = 2e-14 if precision == "double" else 3e-6
     assert float((lines - passes).norm() / passes.norm()) <= tol
+    assert float((auto - passes).norm() / passes.norm()) <= tol
 
 
-@pytest.mark.parametrize("shape,images", [((162, 162), 6), ((243, 96), 6), ((96, 189), 6), ((125, 125), 18), ((512, 48), 1),
+@pytest.mark.parametrize("shape,images", [((162, 162), 6), ((243, 96), 6), ((96, 189), 18), ((125, 125), 18), ((512, 48), 1),
                                           ((48, 512), 1)])
 @pytest.mark.parametrize("precision,tol", [("double", 2e-14), ("mixed", 3e-6)])
 def test_refocus_of_such_sides(shape, images, precision, tol):
